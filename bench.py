@@ -1038,7 +1038,7 @@ def main():
     traffic, traffic_src = profile_traffic(args.level, cells, fmt_bytes)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_src,
-                "kernel": "rbgs_pipelined_kernel<res,sweep> (fused residual + red-black sweep)",
+                "kernel": "rbgs_block_kernel<res,sweep> (fused residual + red-black sweep)",
                 "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_launch_ms,
                 "bytes_per_cell": BYTES_PER_SWEEP_CELL, "uniform_blocks": ublocks,
                 "format_bytes_per_launch": fmt_bytes,

@@ -116,6 +116,97 @@ static __device__ __noinline__ double guide_value(const T* __restrict__ x, int b
   }
 }
 
+// The eight cells (i..i+1, j..j+1, k..k+1) of block blk: nnn, pnn, npn, nnp,
+// npp, pnp, ppn, ppp (first letter: +1 along i, then j, then k).
+template <typename T>
+__device__ __forceinline__ void load8(const T* __restrict__ x, int blk, int i, int j, int k,
+                                      double (&a)[8]) {
+  const T* b = x + (size_t)blk * BLOCK_CELLS + (k * 16 + j) * 8;
+  const int e = ((i + j + k) & 1) << 11, o = e ^ HALF_CELLS, h0 = i >> 1, h1 = (i + 1) >> 1;
+  a[0] = (double)__ldg(b + e + h0);
+  a[1] = (double)__ldg(b + o + h1);
+  a[2] = (double)__ldg(b + o + 8 + h0);
+  a[3] = (double)__ldg(b + o + 128 + h0);
+  a[4] = (double)__ldg(b + e + 136 + h0);
+  a[5] = (double)__ldg(b + e + 128 + h1);
+  a[6] = (double)__ldg(b + e + 8 + h1);
+  a[7] = (double)__ldg(b + o + 136 + h1);
+}
+
+// Guide cell (layer 1) at position p (u + 16 v) of a 2:1 face, in two steps
+// so that several cells' loads can be in flight together; the expressions,
+// and so the bits, are guide_value's.  The face's axis may differ from thread
+// to thread, so the coordinates are chosen by selects: arrays indexed by the
+// axis would live in local memory.
+struct CoarseGuide {  // interpolation from a coarse neighbour (sup.f90:54-120)
+  double a[8], r, s, t;
+  int blk, i, j, k;
+  __device__ __forceinline__ void at(int face, int p, const FaceNbr& nb) {
+    const int axis = face >> 1;
+    int iu, iv, ia;
+    double ru, rv, ra;
+    intp_index((p & 15) + 1 + 16 * nb.so_u, 16, iu, ru);
+    intp_index((p >> 4) + 1 + 16 * nb.so_v, 16, iv, rv);
+    intp_index((face & 1) ? 1 : 32, 16, ia, ra);
+    r = axis == 0 ? ra : ru;
+    s = axis == 0 ? ru : axis == 1 ? ra : rv;
+    t = axis == 2 ? ra : rv;
+    blk = nb.id[0];
+    i = (axis == 0 ? ia : iu) - 1;
+    j = (axis == 0 ? iu : axis == 1 ? ia : iv) - 1;
+    k = (axis == 2 ? ia : iv) - 1;
+  }
+  template <typename T>
+  __device__ __forceinline__ void load(const T* __restrict__ x, int face, int p,
+                                       const FaceNbr& nb) {
+    at(face, p, nb);
+    load8(x, blk, i, j, k, a);
+  }
+  __device__ __forceinline__ double value() const {
+    return (1.0 - t) * ((1.0 - s) * ((1.0 - r) * a[0] + r * a[1]) +
+                        s * ((1.0 - r) * a[2] + r * a[6])) +
+           t * ((1.0 - s) * ((1.0 - r) * a[3] + r * a[5]) +
+                s * ((1.0 - r) * a[4] + r * a[7]));
+  }
+};
+struct FineGuide {  // mean of eight cells of a fine neighbour (sup.f90:122-179)
+  double a[8];
+  int blk, i, j, k;
+  __device__ __forceinline__ void at(int face, int p, const FaceNbr& nb) {
+    const int axis = face >> 1, u = p & 15, v = p >> 4;
+    const int lu = 2 * (u & 7), lv = 2 * (v & 7), la = (face & 1) ? 0 : 14;
+    const int b0 = (v >> 3) ? nb.id[2] : nb.id[0], b1 = (v >> 3) ? nb.id[3] : nb.id[1];
+    blk = (u >> 3) ? b1 : b0;
+    i = axis == 0 ? la : lu;
+    j = axis == 0 ? lu : axis == 1 ? la : lv;
+    k = axis == 2 ? la : lv;
+  }
+  template <typename T>
+  __device__ __forceinline__ void load(const T* __restrict__ x, int face, int p,
+                                       const FaceNbr& nb) {
+    at(face, p, nb);
+    load8(x, blk, i, j, k, a);
+  }
+  __device__ __forceinline__ double value() const {
+    return 0.125 * (a[0] + a[1] + a[2] + a[3] + a[4] + a[5] + a[6] + a[7]);
+  }
+};
+// Storage slot of the cell a same-level guide at position p copies (the
+// neighbour's layer next to the face) or, with own, of the block's own cell
+// that an outer guide is computed from.
+__device__ __forceinline__ int face_slot(int f, int p, bool own) {
+  const int u = p & 15, v = p >> 4, axis = f >> 1;
+  const int a = ((f & 1) != 0) == own ? 15 : 0;
+  return sidx(axis == 0 ? a : u, axis == 0 ? u : axis == 1 ? a : v, axis == 2 ? a : v);
+}
+// Outer guide (layer 1) from the block's own cell x0: bcx.f90 bc_x?_d (5-147)
+// / bc_x?_n (294-436).
+__device__ __forceinline__ double outer_guide(double x0, int face, const BCSet& bc, double dx) {
+  if (bc.type[face] == BC_DIRICHLET) return 2.0 * bc.value[face] - x0;
+  const double xc = bc.value[face] * dx;
+  return (face & 1) ? (x0 + xc) : (x0 - xc);
+}
+
 // Two guide cells (layer 1) of the same face, positions p0 and p1 in
 // [0, 256) (p = v*16 + u), with every load of both issued before any is
 // used: the batched form of guide_value for the pipelined kernels.  Same
@@ -124,76 +215,27 @@ template <typename T>
 __device__ __forceinline__ void guide_pair(const T* __restrict__ x, int blk, int face,
                                            int p0, int p1, const FaceNbr& nb, const BCSet& bc,
                                            double dx, double& v0, double& v1) {
-  const int axis = face >> 1;
-  const bool plus = face & 1;
-  const int ta = (axis == 0) ? 1 : 0, tb = (axis == 2) ? 1 : 2;
-  int g0[3], g1[3];
-  g0[ta] = p0 & 15; g0[tb] = p0 >> 4; g0[axis] = plus ? 16 : -1;
-  g1[ta] = p1 & 15; g1[tb] = p1 >> 4; g1[axis] = plus ? 16 : -1;
-  if (nb.kind == NB_SAME) {
-    g0[axis] = g1[axis] = plus ? 0 : 15;
-    v0 = ld(x, nb.id[0], g0[0], g0[1], g0[2]);
-    v1 = ld(x, nb.id[0], g1[0], g1[1], g1[2]);
-    return;
-  }
   if (nb.kind == NB_COARSE) {
-    int f0[3], f1[3];
-    f0[ta] = g0[ta] + 1 + 16 * nb.so_u; f0[tb] = g0[tb] + 1 + 16 * nb.so_v;
-    f1[ta] = g1[ta] + 1 + 16 * nb.so_u; f1[tb] = g1[tb] + 1 + 16 * nb.so_v;
-    f0[axis] = f1[axis] = plus ? 1 : 32;
-    int i0, j0, k0, i1, j1, k1;
-    double r0, s0, t0, r1, s1, t1;
-    intp_index(f0[0], 16, i0, r0); intp_index(f0[1], 16, j0, s0); intp_index(f0[2], 16, k0, t0);
-    intp_index(f1[0], 16, i1, r1); intp_index(f1[1], 16, j1, s1); intp_index(f1[2], 16, k1, t1);
-    --i0; --j0; --k0; --i1; --j1; --k1;
-    const int c = nb.id[0];
-    const double a0 = ld(x, c, i0, j0, k0), a1 = ld(x, c, i0 + 1, j0, k0);
-    const double a2 = ld(x, c, i0, j0 + 1, k0), a3 = ld(x, c, i0, j0, k0 + 1);
-    const double a4 = ld(x, c, i0, j0 + 1, k0 + 1), a5 = ld(x, c, i0 + 1, j0, k0 + 1);
-    const double a6 = ld(x, c, i0 + 1, j0 + 1, k0), a7 = ld(x, c, i0 + 1, j0 + 1, k0 + 1);
-    const double b0 = ld(x, c, i1, j1, k1), b1 = ld(x, c, i1 + 1, j1, k1);
-    const double b2 = ld(x, c, i1, j1 + 1, k1), b3 = ld(x, c, i1, j1, k1 + 1);
-    const double b4 = ld(x, c, i1, j1 + 1, k1 + 1), b5 = ld(x, c, i1 + 1, j1, k1 + 1);
-    const double b6 = ld(x, c, i1 + 1, j1 + 1, k1), b7 = ld(x, c, i1 + 1, j1 + 1, k1 + 1);
-    // nnn, pnn, npn, nnp, npp, pnp, ppn, ppp = a0..a7
-    v0 = (1.0 - t0) * ((1.0 - s0) * ((1.0 - r0) * a0 + r0 * a1) + s0 * ((1.0 - r0) * a2 + r0 * a6)) +
-         t0 * ((1.0 - s0) * ((1.0 - r0) * a3 + r0 * a5) + s0 * ((1.0 - r0) * a4 + r0 * a7));
-    v1 = (1.0 - t1) * ((1.0 - s1) * ((1.0 - r1) * b0 + r1 * b1) + s1 * ((1.0 - r1) * b2 + r1 * b6)) +
-         t1 * ((1.0 - s1) * ((1.0 - r1) * b3 + r1 * b5) + s1 * ((1.0 - r1) * b4 + r1 * b7));
-    return;
-  }
-  if (nb.kind == NB_FINE) {
-    const int fb0 = nb.id[(g0[ta] >> 3) + 2 * (g0[tb] >> 3)];
-    const int fb1 = nb.id[(g1[ta] >> 3) + 2 * (g1[tb] >> 3)];
-    int l0[3], l1[3];
-    l0[ta] = 2 * (g0[ta] & 7); l0[tb] = 2 * (g0[tb] & 7);
-    l1[ta] = 2 * (g1[ta] & 7); l1[tb] = 2 * (g1[tb] & 7);
-    l0[axis] = l1[axis] = plus ? 0 : 14;
-    const int i0 = l0[0], j0 = l0[1], k0 = l0[2], i1 = l1[0], j1 = l1[1], k1 = l1[2];
-    const double a0 = ld(x, fb0, i0, j0, k0), a1 = ld(x, fb0, i0 + 1, j0, k0);
-    const double a2 = ld(x, fb0, i0, j0 + 1, k0), a3 = ld(x, fb0, i0, j0, k0 + 1);
-    const double a4 = ld(x, fb0, i0, j0 + 1, k0 + 1), a5 = ld(x, fb0, i0 + 1, j0, k0 + 1);
-    const double a6 = ld(x, fb0, i0 + 1, j0 + 1, k0), a7 = ld(x, fb0, i0 + 1, j0 + 1, k0 + 1);
-    const double b0 = ld(x, fb1, i1, j1, k1), b1 = ld(x, fb1, i1 + 1, j1, k1);
-    const double b2 = ld(x, fb1, i1, j1 + 1, k1), b3 = ld(x, fb1, i1, j1, k1 + 1);
-    const double b4 = ld(x, fb1, i1, j1 + 1, k1 + 1), b5 = ld(x, fb1, i1 + 1, j1, k1 + 1);
-    const double b6 = ld(x, fb1, i1 + 1, j1 + 1, k1), b7 = ld(x, fb1, i1 + 1, j1 + 1, k1 + 1);
-    v0 = 0.125 * (a0 + a1 + a2 + a3 + a4 + a5 + a6 + a7);
-    v1 = 0.125 * (b0 + b1 + b2 + b3 + b4 + b5 + b6 + b7);
-    return;
-  }
-  // outer face: bcx.f90 bc_x?_d (5-147) / bc_x?_n (294-436), layer 1
-  g0[axis] = g1[axis] = plus ? 15 : 0;
-  const double x0 = ld(x, blk, g0[0], g0[1], g0[2]);
-  const double x1 = ld(x, blk, g1[0], g1[1], g1[2]);
-  if (bc.type[face] == BC_DIRICHLET) {
-    const double xc = bc.value[face];
-    v0 = 2.0 * xc - x0;
-    v1 = 2.0 * xc - x1;
+    CoarseGuide g0, g1;
+    g0.load(x, face, p0, nb);
+    g1.load(x, face, p1, nb);
+    v0 = g0.value();
+    v1 = g1.value();
+  } else if (nb.kind == NB_FINE) {
+    FineGuide g0, g1;
+    g0.load(x, face, p0, nb);
+    g1.load(x, face, p1, nb);
+    v0 = g0.value();
+    v1 = g1.value();
   } else {
-    const double xc = bc.value[face] * dx;
-    v0 = plus ? (x0 + xc) : (x0 - xc);
-    v1 = plus ? (x1 + xc) : (x1 - xc);
+    const bool own = nb.kind == NB_OUTER;
+    const T* s = x + (size_t)(own ? blk : nb.id[0]) * BLOCK_CELLS;
+    v0 = (double)__ldg(s + face_slot(face, p0, own));
+    v1 = (double)__ldg(s + face_slot(face, p1, own));
+    if (own) {
+      v0 = outer_guide(v0, face, bc, dx);
+      v1 = outer_guide(v1, face, bc, dx);
+    }
   }
 }
 

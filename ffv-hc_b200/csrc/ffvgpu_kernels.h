@@ -21,24 +21,27 @@ struct KCtx {
   int nb;
   int first;
   uint64_t wait_ns;    // limit of every bounded device wait (ffvgpu_pool_set_wait_limit)
-  // [blocks][8] uniform records of A (launch_pack_stream, launch_urec), or
+  // [blocks][8] uniform records of A (launch_urec), or
   // null: every block streams all its coefficients
   const double* urec;
 };
 
-// Fused residual + red-black sweep over the coefficient stream (rbgs_pipelined.cu).
+// Where a pass takes its blocks' guide layers from: stored (gin [blk][face][p]),
+// the neighbours' interiors, or the neighbours' interiors with what the sweep
+// before pushed into gin.
+enum class RbgsGuides { STORED, PULL, PUSHED };
+// Fused residual + red-black sweep (rbgs_block.cu); C.urec must be set.  A
+// sweep with gout pushes guides for the next pass into it (PUSHED).
 // pdl: launched as a programmatic dependent of the previous kernel on the
-// stream, which must then be a pass of this kernel (it overlaps that pass's
-// tail: its coefficient prefetch runs before the dependency wait).
+// stream, which must then be a pass of this kernel.  order: the C.nb blocks in
+// the order the grid takes them (null: block order); results do not depend on it.
 void launch_rbgs(cudaStream_t s, const KCtx& C, bool res, bool sweep, const double* xin,
-                 double* xout, const double* stream, const double* gst, double omega,
-                 double* partials, SolveState* st, int fin, int iter, bool pdl = false);
-// Packs A and b into the sweep's coefficient stream and writes each block's
-// uniform record urec[blk][8] (Ap..At of cell 0, then 1.0 when every cell has
-// those seven coefficients, else 0.0), adding the uniform blocks to *ucount.
-void launch_pack_stream(cudaStream_t s, int nb, const double* A, const double* b, double* stream,
-                        double* urec, int32_t* ucount);
-// The uniform records alone (the record format of launch_pack_stream).
+                 double* xout, const double* A, const double* b, RbgsGuides from,
+                 const double* gin, double* gout, double omega, double* partials, SolveState* st,
+                 int fin, int iter, bool pdl = false, const int32_t* order = nullptr);
+// Each block's uniform record urec[blk][8] (Ap..At of cell 0, then 1.0 when
+// every cell has those seven coefficients, else 0.0), adding the uniform
+// blocks to *ucount.
 void launch_urec(cudaStream_t s, int nb, const double* A, double* urec, int32_t* ucount);
 // Jacobi sweep from the zero field (the preconditioner's first pass); a
 // block with a set uniform record (C.urec) reads its seven coefficients from

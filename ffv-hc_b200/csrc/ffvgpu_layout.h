@@ -32,11 +32,6 @@ constexpr int BLOCK_CELLS = 4096; // 16^3
 constexpr int HALF_CELLS = 2048;  // cells of one colour
 constexpr int FACE_CELLS = 256;   // 16^2
 constexpr int THREADS = 256;      // threads per CTA of every block kernel
-// Coefficient stream of the red-black sweep: per block 16 chunks (colour c,
-// plane pair m -> chunk c*8 + m), each holding Ap, Aw, Ae, As, An, Ab, At, b
-// of its 256 cells back to back (16 KB), so one bulk copy moves a chunk.
-constexpr int STREAM_CHUNK = 8 * 256;
-constexpr int STREAM_BLOCK = 16 * STREAM_CHUNK;
 // Default limit of every bounded device wait (a pool setting,
 // ffvgpu_pool_set_wait_limit): a wait that has not completed after it gives
 // up and the solve reports a timeout.
@@ -87,6 +82,7 @@ struct SolveState {
   double best;       // mixed form: smallest residual of the current cycle
   double growth;     // mixed form: restart when the residual exceeds growth * best (0: never)
   double scale;      // RBGS_WithFixedAverage: the cell count the sum is divided by
+  uint32_t work;     // RBGS pass: blocks handed out beyond each CTA's first
   int32_t max_cycle; // mixed form: restart after this many iterations of a cycle (0: never)
   int32_t ublocks;   // mixed form: blocks whose seven coefficients are the same in every cell
 };

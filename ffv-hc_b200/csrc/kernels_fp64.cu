@@ -696,29 +696,18 @@ fold_bc_kernel(KCtx C, double* __restrict__ A, double* __restrict__ bvec) {
   }
 }
 
-// A (7 arrays) and b -> the sweep's coefficient stream (STREAM_BLOCK per block).
-// Without STREAM only the uniform records are written.
-template <bool STREAM>
+// The uniform records of A (launch_urec): a block is uniform when all seven
+// coefficients of every cell are bitwise equal to cell 0's.
 __global__ void __launch_bounds__(THREADS)
-pack_stream_kernel(const double* __restrict__ A, const double* __restrict__ b,
-                   double* __restrict__ stream, double* __restrict__ urec,
-                   int32_t* __restrict__ ucount) {
+urec_kernel(const double* __restrict__ A, double* __restrict__ urec,
+            int32_t* __restrict__ ucount) {
   const int blk = blockIdx.x, tid = threadIdx.x;
   const double* Ab = A + (size_t)blk * 7 * BLOCK_CELLS;
-  double* sb = STREAM ? stream + (size_t)blk * STREAM_BLOCK : nullptr;
   bool same = true;
-  for (int m = 0; m < 16; ++m) {
-    const int s = tid + THREADS * m;  // chunk m, cell tid
-    double* dst = STREAM ? sb + (size_t)m * STREAM_CHUNK + tid : nullptr;
-    for (int a = 0; a < 7; ++a) {
-      const double v = Ab[(size_t)a * BLOCK_CELLS + s];
-      if (STREAM) dst[a * 256] = v;
-      same = same && __double_as_longlong(v) == __double_as_longlong(Ab[(size_t)a * BLOCK_CELLS]);
-    }
-    if (STREAM) dst[7 * 256] = b[(size_t)blk * BLOCK_CELLS + s];
-  }
-  // a uniform block (all seven coefficients bitwise equal to cell 0's): the
-  // sweep kernel copies only b of its stream and takes Ap..At from here
+  for (int m = 0; m < 16; ++m)
+    for (int a = 0; a < 7; ++a)
+      same = same && __double_as_longlong(Ab[(size_t)a * BLOCK_CELLS + tid + THREADS * m]) ==
+                         __double_as_longlong(Ab[(size_t)a * BLOCK_CELLS]);
   same = __syncthreads_and(same);
   if (tid < 8) urec[(size_t)blk * 8 + tid] = tid < 7 ? Ab[(size_t)tid * BLOCK_CELLS] : (same ? 1.0 : 0.0);
   if (tid == 0 && same) atomicAdd(ucount, 1);
@@ -810,12 +799,8 @@ void launch_assemble(cudaStream_t s, const KCtx& C, const double* ux, const doub
   assemble_kernel<<<C.nb, THREADS, 0, s>>>(C, ux, uy, uz, gux, guy, guz, cut, flags, A, b, vface,
                                            rhof, dt, field_stride);
 }
-void launch_pack_stream(cudaStream_t s, int nb, const double* A, const double* b, double* stream,
-                        double* urec, int32_t* ucount) {
-  pack_stream_kernel<true><<<nb, THREADS, 0, s>>>(A, b, stream, urec, ucount);
-}
 void launch_urec(cudaStream_t s, int nb, const double* A, double* urec, int32_t* ucount) {
-  pack_stream_kernel<false><<<nb, THREADS, 0, s>>>(A, nullptr, nullptr, urec, ucount);
+  urec_kernel<<<nb, THREADS, 0, s>>>(A, urec, ucount);
 }
 void launch_fill(cudaStream_t s, int nb, double* x, size_t stride, double* g, double value) {
   fill_kernel<<<nb, THREADS, 0, s>>>(x, stride, g, value);

@@ -184,24 +184,6 @@ ffvgpu_status require_system(ffvgpu_pool* P) {
   return field_ptr(P, FFVGPU_FIELD_X, true, &xp, &st, nullptr);
 }
 
-// Repacks A and b into the sweep's coefficient stream when they changed.
-ffvgpu_status ensure_stream(ffvgpu_pool* P) {
-  ffvgpu_status s;
-  if ((s = dalloc_t(P, &P->coef, (size_t)P->nb * STREAM_BLOCK)) ||
-      (s = dalloc_t(P, &P->urec, (size_t)P->nb * 8)) || (s = dalloc_t(P, &P->ucount_d, 1)))
-    return s;
-  if (P->stream_version != P->sys_version) {
-    CK(cudaMemsetAsync(P->ucount_d, 0, sizeof(int32_t), P->stream));
-    launch_pack_stream(P->stream, P->nb, P->A, P->b, P->coef, P->urec, P->ucount_d);
-    CK(cudaGetLastError());
-    CK(download_sync(P, &P->ucount_h, P->ucount_d, sizeof(int32_t)));
-    P->stream_version = P->sys_version;
-    P->urec_version = P->sys_version;
-    P->ucount_version = P->sys_version;
-  }
-  return FFVGPU_OK;
-}
-
 // The uniform records of A (KCtx::urec) when A changed.
 ffvgpu_status ensure_urec(ffvgpu_pool* P) {
   ffvgpu_status s;
@@ -214,6 +196,16 @@ ffvgpu_status ensure_urec(ffvgpu_pool* P) {
     P->urec_version = P->sys_version;
   }
   return FFVGPU_OK;
+}
+
+// The guide buffers that RBGS passes push into, for a neighbour table in which
+// every face is the other side's neighbour too (a shard's halo faces are not).
+ffvgpu_status ensure_push(ffvgpu_pool* P) {
+  if (!P->nbr_mutual) return FFVGPU_OK;
+  ffvgpu_status s;
+  const size_t n = (size_t)P->nb * 6 * FACE_CELLS;
+  if ((s = dalloc_t(P, &P->gpush[0], n))) return s;
+  return dalloc_t(P, &P->gpush[1], n);
 }
 
 // The FP64 solvers' pipelined A*x over the pool as one instance: its block
@@ -234,11 +226,6 @@ ffvgpu_status ensure_kpipe(ffvgpu_pool* P) {
     h[(size_t)2 * nb + 2] = nb;  // count; blk_inst and first stay 0
     CK(upload(P, P->kraw, h.data(), sizeof(int32_t) * ((size_t)nb + 1)));
     CK(upload(P, P->kpipe + 1 + nb, h.data() + 1 + nb, sizeof(int32_t) * ((size_t)nb + 2)));
-    if (!P->grid_mvpipe) {
-      int a, b, c, d, e;
-      mx_grid_sizes(P->m_threads, &a, &b, &c, &d, &e);
-      P->grid_mvpipe = e;
-    }
     P->kpipe_version = 0;
     P->kpipe_ready = true;
   }
@@ -275,12 +262,21 @@ MixCtx krylov_mix_ctx(const ffvgpu_pool* P, int fin) {
   return C;
 }
 
+// CTAs of the pipelined kernel.
+int krylov_grid(ffvgpu_pool* P) {
+  if (!P->grid_mvpipe) {
+    int a, b, c, d, e;
+    mx_grid_sizes(P->m_threads, &a, &b, &c, &d, &e);
+    P->grid_mvpipe = e;
+  }
+  return P->grid_cap > 0 && P->grid_cap < P->grid_mvpipe ? P->grid_cap : P->grid_mvpipe;
+}
+
 // q = A x and q.w (fin FIN_BI_QR0 or FIN_CG_QP), or with t.t as well
 // (FIN_BI_TS, then FIN_BI_TT) when 'two'.
 void krylov_matvec(ffvgpu_pool* P, const double* x, double* q, const double* w, int fin,
                    bool two) {
-  int grid = P->grid_mvpipe;
-  if (P->grid_cap > 0 && P->grid_cap < grid) grid = P->grid_cap;
+  const int grid = krylov_grid(P);
   launch_mx_matvec(P->stream, krylov_mix_ctx(P, fin), grid, two ? 2 : 1, 0, 0, x, P->A, q, w,
                    true);
 }
@@ -289,8 +285,7 @@ void krylov_matvec(ffvgpu_pool* P, const double* x, double* q, const double* w, 
 // with dot also b.y (FIN_CG_RR1).
 void krylov_jacobi(ffvgpu_pool* P, const double* x, double* y, const double* b, double omega,
                    bool dot) {
-  int grid = P->grid_mvpipe;
-  if (P->grid_cap > 0 && P->grid_cap < grid) grid = P->grid_cap;
+  const int grid = krylov_grid(P);
   launch_jacobi_pipe(P->stream, krylov_mix_ctx(P, dot ? FIN_CG_RR1 : 0), grid, dot, x, P->A, b,
                      y, omega);
 }
@@ -377,6 +372,23 @@ ffvgpu_status explicit_neighbors(ffvgpu_pool* P, const ffvgpu_grid_desc* d) {
   return FFVGPU_OK;
 }
 
+// Whether every face record is matched by the neighbour's record of the same face.
+bool mutual_neighbors(const std::vector<FaceNbr>& t, int nb) {
+  for (int b = 0; b < nb; ++b)
+    for (int f = 0; f < 6; ++f) {
+      const FaceNbr& F = t[(size_t)b * 6 + f];
+      for (int q = 0; q < (F.kind == NB_FINE ? 4 : F.kind == NB_OUTER ? 0 : 1); ++q) {
+        const FaceNbr& O = t[(size_t)F.id[q] * 6 + (f ^ 1)];
+        const bool ok = F.kind == NB_SAME   ? O.kind == NB_SAME && O.id[0] == b
+                        : F.kind == NB_FINE ? O.kind == NB_COARSE && O.id[0] == b &&
+                                                  O.so_u == (q & 1) && O.so_v == (q >> 1)
+                                            : O.kind == NB_FINE && O.id[F.so_u + 2 * F.so_v] == b;
+        if (!ok) return false;
+      }
+    }
+  return true;
+}
+
 ffvgpu_status solve_status(const SolveState& h, const ffvgpu_iter_params* prm, int N, int count) {
   if (h.status == 3) {
     g_last_error = timeout_message(h.timeout_where);
@@ -393,6 +405,14 @@ ffvgpu_status solve_status(const SolveState& h, const ffvgpu_iter_params* prm, i
 int64_t interior_bytes(const ffvgpu_pool* P, int words) {
   return (int64_t)P->nb * (int64_t)BC * 8 * words;
 }
+// The count of uniform blocks, read back once per assembled A.
+ffvgpu_status read_ucount(ffvgpu_pool* P) {
+  if (P->ucount_version != P->sys_version) {
+    CK(download_sync(P, &P->ucount_h, P->ucount_d, sizeof(int32_t)));
+    P->ucount_version = P->sys_version;
+  }
+  return FFVGPU_OK;
+}
 // Bytes of one pass of the red-black kernel: 'words' per cell (10 for a
 // sweep with its residual, 9 for a residual alone) in a block that streams
 // its coefficients, 'words' - 7 in a uniform block (b and x only).
@@ -403,12 +423,10 @@ int64_t rbgs_pass_bytes(const ffvgpu_pool* P, int words) {
 // Bytes the kernels of an FP64 Krylov solve moved: 'words' values per cell
 // over every block, less 'coef' per-cell coefficient words in each uniform
 // block (the Jacobi and A*x kernels read its seven coefficients once from
-// its record).  The uniform count is read back once per assembled A.
+// its record).
 ffvgpu_status krylov_bytes(ffvgpu_pool* P, int64_t words, int64_t coef, int64_t* bytes) {
-  if (P->ucount_version != P->sys_version) {
-    CK(download_sync(P, &P->ucount_h, P->ucount_d, sizeof(int32_t)));
-    P->ucount_version = P->sys_version;
-  }
+  ffvgpu_status s = read_ucount(P);
+  if (s != FFVGPU_OK) return s;
   *bytes = ((int64_t)P->nb * words - (int64_t)P->ucount_h * coef) * (int64_t)BC * 8;
   return FFVGPU_OK;
 }
@@ -489,6 +507,7 @@ ffvgpu_status ffvgpu_pool_create(const ffvgpu_grid_desc* d, ffvgpu_pool** out) {
     delete P;
     return s;
   }
+  P->nbr_mutual = mutual_neighbors(P->nbr_h, P->nb);
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
     delete P;
@@ -524,10 +543,10 @@ void ffvgpu_pool_destroy(ffvgpu_pool* P) {
   if (P->stream) cudaStreamSynchronize(P->stream);
   if (P->own_stream) cudaStreamSynchronize(P->own_stream);
   release_instances(P);
-  void* ptrs[] = {P->x[0], P->x[1], P->gx, P->A, P->coef, P->urec, P->ucount_d, P->b, P->u[0], P->u[1], P->u[2],
+  void* ptrs[] = {P->x[0], P->x[1], P->gx, P->A, P->urec, P->ucount_d, P->b, P->u[0], P->u[1], P->u[2],
                   P->gu[0], P->gu[1], P->gu[2], P->cut, P->vface, P->lapp, P->flags, P->r,
                   P->p, P->q, P->z[0], P->z[1], P->r0, P->sv, P->tv, P->zb[0], P->zb[1],
-                  P->partials, P->st, P->hist_d, P->kpipe, P->kraw, P->kpart,
+                  P->partials, P->st, P->hist_d, P->kpipe, P->kraw, P->kpart, P->gpush[0], P->gpush[1],
                   P->stage, P->nbr_d, P->dx_d};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -817,9 +836,9 @@ ffvgpu_status ffvgpu_calc_r2(ffvgpu_pool* P, double* rr) {
   ffvgpu_status s;
   if ((s = require_system(P))) return s;
   if ((s = reset_state(P, 0.0, 0, nullptr))) return s;
-  if ((s = ensure_stream(P))) return s;
-  launch_rbgs(P->stream, P->ctx(P->bc_p), true, false, P->x[P->xcur], nullptr, P->coef, P->gx,
-              0.0, P->partials, P->st, FIN_STORE, 0);
+  if ((s = ensure_urec(P))) return s;
+  launch_rbgs(P->stream, P->ctx(P->bc_p), true, false, P->x[P->xcur], nullptr, P->A, P->b,
+              RbgsGuides::STORED, P->gx, nullptr, 0.0, P->partials, P->st, FIN_STORE, 0);
   CK(cudaGetLastError());
   SolveState h;
   if ((s = read_state(P, &h))) return s;
@@ -838,9 +857,10 @@ ffvgpu_status ffvgpu_rbgs_sweep(ffvgpu_pool* P, double omega) {
   ffvgpu_status s;
   if ((s = require_system(P))) return s;
   if ((s = reset_state(P, 0.0, 0, nullptr))) return s;
-  if ((s = ensure_stream(P))) return s;
+  if ((s = ensure_urec(P))) return s;
   launch_rbgs(P->stream, P->ctx(P->bc_p), false, true, P->x[P->xcur], P->x[1 - P->xcur],
-              P->coef, P->gx, omega, P->partials, P->st, FIN_STORE, 0);
+              P->A, P->b, RbgsGuides::STORED, P->gx, nullptr, omega, P->partials, P->st,
+              FIN_STORE, 0);
   P->xcur = 1 - P->xcur;
   launch_exchange(P->stream, P->ctx(P->bc_p), P->x[P->xcur], P->gx);
   CK(cudaGetLastError());
@@ -873,20 +893,23 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
     return FFVGPU_OK;
   }
   if ((s = ensure_hist(P, N))) return s;
-  if ((s = ensure_stream(P))) return s;
+  if ((s = ensure_urec(P))) return s;
   if ((s = reset_state(P, prm->epsilon, N, P->hist_d))) return s;
+  if ((s = ensure_push(P))) return s;
+  const RbgsGuides from = P->gpush[0] ? RbgsGuides::PUSHED : RbgsGuides::PULL;
+  if ((s = ensure_kpipe(P))) return s;
+  const int32_t* order = P->kpipe + 1;
   const KCtx C = P->ctx(P->bc_p);
   const int every = prm->check_every > 0 ? prm->check_every : 32;
   const bool poll = prm->epsilon > 0.0;
   CK(cudaEventRecord(P->ev0, P->stream));
   launch_dot(P->stream, C, P->b, P->b, P->partials, P->st, FIN_BB, 0);
   int launches = 1;
-  int64_t bytes = interior_bytes(P, 2);
   const int c0 = P->xcur;
-  launch_rbgs(P->stream, C, false, true, P->x[c0], P->x[1 - c0], P->coef, P->gx, prm->omega,
-              P->partials, P->st, FIN_RBGS, 0);
+  launch_rbgs(P->stream, C, false, true, P->x[c0], P->x[1 - c0], P->A, P->b,
+              RbgsGuides::STORED, P->gx, P->gpush[0], prm->omega, P->partials, P->st, FIN_RBGS, 0,
+              false, order);
   launches++;
-  bytes += rbgs_pass_bytes(P, 10);
   CK(cudaEventRecord(P->ev2, P->stream));
   int swept = 0;
   // Each pass is a programmatic dependent of the pass before it (it
@@ -894,12 +917,12 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   // poll or a timing event sits between them.
   bool polled_last = true;
   for (int n = 2; n <= N; ++n) {
-    launch_rbgs(P->stream, C, true, true, P->x[(c0 + n - 1) & 1], P->x[(c0 + n) & 1], P->coef,
-                nullptr, prm->omega, P->partials, P->st, FIN_RBGS, n - 1, !polled_last);
+    launch_rbgs(P->stream, C, true, true, P->x[(c0 + n - 1) & 1], P->x[(c0 + n) & 1], P->A, P->b,
+                from, P->gpush[n & 1], P->gpush[(n + 1) & 1], prm->omega, P->partials, P->st,
+                FIN_RBGS, n - 1, !polled_last, order);
     polled_last = false;
     swept++;
     launches++;
-    bytes += rbgs_pass_bytes(P, 10);
     if (poll && (n % every) == 0) {
       bool done = false;
       if ((s = poll_done(P, &done))) return s;
@@ -908,8 +931,9 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
     }
   }
   CK(cudaEventRecord(P->ev3, P->stream));
-  launch_rbgs(P->stream, C, true, false, P->x[(c0 + N) & 1], nullptr, P->coef, nullptr,
-              prm->omega, P->partials, P->st, FIN_RBGS, N, false);
+  launch_rbgs(P->stream, C, true, false, P->x[(c0 + N) & 1], nullptr, P->A, P->b,
+              from, P->gpush[(N + 1) & 1], nullptr, prm->omega, P->partials, P->st, FIN_RBGS, N,
+              false, order);
   launches++;
   CK(cudaEventRecord(P->ev1, P->stream));
   CK(cudaGetLastError());
@@ -920,7 +944,8 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   // (the solve ran to countMax, or converged on its last residual) iterate N
   const int m = early ? h.count : N;
   // passes that ran: sweeps 1..min(m+1, N), residual-only pass only at the end
-  bytes = interior_bytes(P, 2) + rbgs_pass_bytes(P, 10) * (early ? (m + 1) : N) +
+  if ((s = read_ucount(P))) return s;
+  const int64_t bytes = interior_bytes(P, 2) + rbgs_pass_bytes(P, 10) * (early ? (m + 1) : N) +
           (early ? 0 : rbgs_pass_bytes(P, 9));
   P->xcur = (c0 + m) & 1;
   launch_exchange(P->stream, C, P->x[P->xcur], P->gx);
@@ -966,7 +991,7 @@ ffvgpu_status ffvgpu_solve_rbgs_fixed_average(ffvgpu_pool* P, const ffvgpu_iter_
     if (res) *res = R;
     return FFVGPU_OK;
   }
-  if ((s = ensure_hist(P, N)) || (s = ensure_stream(P))) return s;
+  if ((s = ensure_hist(P, N)) || (s = ensure_urec(P))) return s;
   SolveState h0;
   std::memset(&h0, 0, sizeof(h0));
   h0.eps = prm->epsilon;
@@ -981,22 +1006,22 @@ ffvgpu_status ffvgpu_solve_rbgs_fixed_average(ffvgpu_pool* P, const ffvgpu_iter_
   const bool poll = prm->epsilon > 0.0;
   CK(cudaEventRecord(P->ev0, P->stream));
   launch_dot(P->stream, C, P->b, P->b, P->partials, P->st, FIN_BB, 0);
-  int launches = 1;
-  int64_t bytes = interior_bytes(P, 2);
+  int launches = 1, passes = 0;
   const int c0 = P->xcur;
   int cur = c0;
   for (int n = 1; n <= N; ++n) {
     // once the solve has stopped these kernels return at entry: the iterate
     // kept is the one of the stopping iteration (below)
-    launch_rbgs(P->stream, C, false, true, P->x[cur], P->x[1 - cur], P->coef,
-                n == 1 ? P->gx : nullptr, prm->omega, P->partials, P->st, FIN_STORE, n);
+    launch_rbgs(P->stream, C, false, true, P->x[cur], P->x[1 - cur], P->A, P->b,
+                n == 1 ? RbgsGuides::STORED : RbgsGuides::PULL, n == 1 ? P->gx : nullptr, nullptr,
+                prm->omega, P->partials, P->st, FIN_STORE, n);
     cur = 1 - cur;
     launch_sum(P->stream, C, P->x[cur], P->partials, P->st, FIN_FA_SHIFT);
     launch_shift(P->stream, C, P->x[cur], P->st);
-    launch_rbgs(P->stream, C, true, false, P->x[cur], nullptr, P->coef, nullptr, prm->omega,
-                P->partials, P->st, FIN_RBGS, n);
+    launch_rbgs(P->stream, C, true, false, P->x[cur], nullptr, P->A, P->b,
+                RbgsGuides::PULL, nullptr, nullptr, prm->omega, P->partials, P->st, FIN_RBGS, n);
     launches += 4;
-    bytes += rbgs_pass_bytes(P, 10) + interior_bytes(P, 1 + 2) + rbgs_pass_bytes(P, 9);
+    passes++;
     if (poll && (n % every) == 0) {
       bool done = false;
       if ((s = poll_done(P, &done))) return s;
@@ -1017,7 +1042,10 @@ ffvgpu_status ffvgpu_solve_rbgs_fixed_average(ffvgpu_pool* P, const ffvgpu_iter_
   R.count = h.count;
   R.residual = h.residual;
   R.elapsed_ms = ms;
-  R.bytes_moved = bytes;
+  if ((s = read_ucount(P))) return s;
+  R.bytes_moved = interior_bytes(P, 2) + passes * (rbgs_pass_bytes(P, 10) +
+                                                   interior_bytes(P, 1 + 2) +
+                                                   rbgs_pass_bytes(P, 9));
   R.kernel_launches = launches + 1;
   if (prm->history) {
     const int nh = (h.count >= 1 && h.count <= N) ? h.count : N;
@@ -1271,13 +1299,13 @@ ffvgpu_status ffvgpu_rbgs_pass(ffvgpu_pool* P, int32_t blocks, int32_t residual,
   cudaSetDevice(P->device);
   ffvgpu_status s;
   if ((s = require_system(P))) return s;
-  if ((s = ensure_stream(P))) return s;
+  if ((s = ensure_urec(P))) return s;
   if ((s = reset_state(P, 0.0, 0, nullptr))) return s;
   KCtx C = P->ctx(P->bc_p);
   C.nb = blocks;
   const int c = P->xcur;
-  launch_rbgs(P->stream, C, res, swp, P->x[c], swp ? P->x[1 - c] : nullptr, P->coef,
-              st ? P->gx : nullptr, omega, P->partials, P->st, FIN_STORE, 0);
+  launch_rbgs(P->stream, C, res, swp, P->x[c], swp ? P->x[1 - c] : nullptr, P->A, P->b,
+              st ? RbgsGuides::STORED : RbgsGuides::PULL, st ? P->gx : nullptr, nullptr, omega, P->partials, P->st, FIN_STORE, 0);
   CK(cudaGetLastError());
   if (swp) P->xcur = 1 - c;
   SolveState h;

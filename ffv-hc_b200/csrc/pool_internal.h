@@ -92,12 +92,10 @@ struct ffvgpu_pool {
   int xcur = 0;
   double* gx = nullptr;  // stored first guide layer of x
   double* A = nullptr;   // [nb][7][4096]
-  double* coef = nullptr;         // sweep coefficient stream [nb][STREAM_BLOCK]
-  double* urec = nullptr;         // [nb][8] uniform records of the stream (launch_pack_stream)
-  int32_t* ucount_d = nullptr;    // uniform blocks of the stream
-  int32_t ucount_h = 0;           // the same, read after each repack
+  double* urec = nullptr;         // [nb][8] uniform records of A (launch_urec)
+  int32_t* ucount_d = nullptr;    // uniform blocks
+  int32_t ucount_h = 0;           // the same, read back for a solve's byte count
   int64_t sys_version = 1;        // bumped whenever A or b change
-  int64_t stream_version = 0;     // sys_version the stream was packed from
   int64_t urec_version = 0;       // sys_version the uniform records come from
   int64_t ucount_version = 0;     // sys_version ucount_h was read back for
   double* b = nullptr;
@@ -130,6 +128,8 @@ struct ffvgpu_pool {
   int32_t* kraw = nullptr;
   double* kpart = nullptr;
   int64_t kpipe_version = 0;  // sys_version the list was ordered for
+  bool nbr_mutual = false;  // every face is the other side's neighbour too
+  double* gpush[2] = {nullptr, nullptr};  // [nb][6][256] guides pushed by RBGS passes
   bool kpipe_ready = false;   // all three allocated and the tables uploaded
 
   // instances: a pool made from one grid is instance 0 over every block; a

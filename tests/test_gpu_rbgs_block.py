@@ -1,0 +1,42 @@
+"""The RBGS pass where its launch and its arithmetic change form: block counts
+around one and two blocks per SM (and one block alone), where the grid deals
+out further blocks as CTAs free up; and right-hand sides whose quotients the
+fast division by a uniform block's diagonal must leave to '/' (zeros, values
+near the ends of the exponent range, infinities).  Bit equality with the
+oracle throughout."""
+import numpy as np
+import pytest
+
+import ffvgpu
+from helpers import VC, assert_bitwise, device_problem, interior, problem
+
+pytestmark = pytest.mark.gpu
+
+
+def compare(g, inp, O, count, scale=None):
+    P = device_problem(g, inp)
+    if scale is not None:
+        with np.errstate(all="ignore"):
+            b = P.download("B", VC) * scale
+        P.upload("B", b, VC)
+        O.field("B")[...] = b
+    P.fill("X", 0.0)
+    O.field("X")[...] = 0.0
+    ro = O.solve_rbgs(1.1, count, 0.0)
+    rg = P.solve_rbgs(1.1, count, 0.0)
+    assert_bitwise(rg["history"], ro["history"], "history")
+    assert_bitwise(interior(P.download("X", VC)), interior(O.field("X")), "x")
+    P.close()
+    O.close()
+
+
+@pytest.mark.parametrize("level,root,radius", [
+    (0, (1, 1, 1), 0.5), (0, (37, 4, 1), 0.5), (0, (149, 1, 1), 0.5), (0, (37, 8, 1), 0.5),
+    (0, (27, 11, 1), 0.5), (0, (8, 8, 8), 3.0), (2, (3, 2, 2), 0.9), (4, (4, 2, 2), 0.55)])
+def test_block_counts(level, root, radius):
+    compare(*problem(level, root_grid=root, radius=radius), 4)
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.0, 1e-310, 1e-290, 1e-200, 1e200, 1e290, np.inf])
+def test_quotients_at_the_ends_of_the_range(scale):
+    compare(*problem(2), 3, scale)
