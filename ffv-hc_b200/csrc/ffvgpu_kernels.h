@@ -50,11 +50,25 @@ void launch_jacobi(cudaStream_t s, const KCtx& C, bool dot, double* xout, const 
                    const double* b, double omega, double* partials, SolveState* st);
 void launch_calc_r(cudaStream_t s, const KCtx& C, const double* x, const double* gst,
                    const double* A, const double* b, double* r, SolveState* st);
-void launch_p_update(cudaStream_t s, const KCtx& C, const double* z, double* p, int first,
-                     SolveState* st);
-// p = r on the first iteration of a cycle (st->cycle == 1), else the update.
-void launch_bicg_p(cudaStream_t s, const KCtx& C, const double* r, double* p, const double* q,
-                   SolveState* st);
+// Cell-wise steps of the Krylov solvers (krylov_block.cu), with the Jacobi pass
+// from zero on the vector formed (C.urec must be set) into z unless z is null,
+// the guides of z (launch_cg_p: of p) pushed into gout unless that is null.
+// p = r (and r0 = r) on the first iteration of a cycle (st->cycle == 1), else the update.
+void launch_bicg_p(cudaStream_t s, const KCtx& C, double* r, double* p, double* q, double* r0,
+                   const double* A, double* z, double omega, double* gout, SolveState* st);
+void launch_bicg_s(cudaStream_t s, const KCtx& C, double* sv, double* q, double* r,
+                   const double* A, double* z, double omega, double* gout, SolveState* st);
+// x, r, the residual of iteration iter, and DOT(r, r0) of the next (partials [2][nb]).
+void launch_bicg_update(cudaStream_t s, const KCtx& C, double* x, double* pz, double* sz,
+                        double* r, double* t, double* sv, double* r0, double* partials,
+                        SolveState* st, int iter);
+void launch_jacobi_zero(cudaStream_t s, const KCtx& C, double* r, const double* A, double* z,
+                        double omega, double* gout, SolveState* st);
+void launch_cg_p(cudaStream_t s, const KCtx& C, double* z, double* p, double* gout,
+                 SolveState* st, int iter);
+void launch_cg_update(cudaStream_t s, const KCtx& C, double* x, double* p, double* r, double* q,
+                      const double* A, double* z, double omega, double* gout, double* partials,
+                      SolveState* st, int iter);
 // Sum of x over the interior (finaliser fin); x += st->alpha.
 void launch_sum(cudaStream_t s, const KCtx& C, const double* x, double* partials, SolveState* st,
                 int fin);
@@ -62,13 +76,6 @@ void launch_shift(cudaStream_t s, const KCtx& C, double* x, SolveState* st);
 // r.r0 (setting r0 = r first on the first iteration of a cycle).
 void launch_dot_rr0(cudaStream_t s, const KCtx& C, const double* r, double* r0, double* partials,
                     SolveState* st, int fin, int iter);
-void launch_axpyz(cudaStream_t s, const KCtx& C, double* z, const double* x, const double* y,
-                  SolveState* st);
-void launch_bicg_update(cudaStream_t s, const KCtx& C, double* x, const double* pz,
-                        const double* sz, double* r, const double* t, const double* sv,
-                        double* partials, SolveState* st, int iter);
-void launch_cg_update(cudaStream_t s, const KCtx& C, double* x, const double* p, double* r,
-                      const double* q, double* partials, SolveState* st, int iter);
 void launch_dot(cudaStream_t s, const KCtx& C, const double* x, const double* y,
                 double* partials, SolveState* st, int fin, int iter);
 void launch_exchange(cudaStream_t s, const KCtx& C, const double* x, double* g);

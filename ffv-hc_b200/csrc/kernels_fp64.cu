@@ -221,104 +221,6 @@ calc_r_kernel(KCtx C, const double* __restrict__ x, const double* __restrict__ g
   }
 }
 
-// p = z (first iteration, copy) or p = z + beta*p (xpay, blas.f90:363-395).
-__global__ void __launch_bounds__(THREADS)
-p_update_kernel(const double* __restrict__ z, double* __restrict__ p, int first, SolveState* st) {
-  if (solve_done(st)) return;
-  const double beta = st->beta;
-  const size_t base = (size_t)blockIdx.x * BLOCK_CELLS;
-#pragma unroll 4
-  for (int m = 0; m < 16; ++m) {
-    const size_t s = base + threadIdx.x + THREADS * m;
-    p[s] = first ? z[s] : (z[s] + beta * p[s]);
-  }
-}
-
-// BiCGSTAB p update (FFVILS.h:853-871): first iteration p = r (copy); after
-// it AXPY(p, q_, -gamma) then XPAY(p, r, beta), i.e. per cell
-// t = p + (-gamma)*q_ ; p = r + beta*t (blas.f90:329-395).
-__global__ void __launch_bounds__(THREADS)
-bicg_p_kernel(const double* __restrict__ r, double* __restrict__ p, const double* __restrict__ q,
-              SolveState* st) {
-  if (solve_done(st)) return;
-  const double beta = st->beta, mgamma = -st->gamma;
-  const bool first = st->cycle == 1;  // iteration 1, or the first after a restart
-  const size_t base = (size_t)blockIdx.x * BLOCK_CELLS;
-#pragma unroll 4
-  for (int m = 0; m < 16; ++m) {
-    const size_t s = base + threadIdx.x + THREADS * m;
-    if (first) {
-      p[s] = r[s];
-    } else {
-      const double t = p[s] + mgamma * q[s];
-      p[s] = r[s] + beta * t;
-    }
-  }
-}
-
-// AXPYZ (blas.f90:397-430): z = a*x + y with a = -alpha (FFVILS.h:898-903).
-__global__ void __launch_bounds__(THREADS)
-axpyz_kernel(double* __restrict__ z, const double* __restrict__ x, const double* __restrict__ y,
-             SolveState* st) {
-  if (solve_done(st)) return;
-  const double a = -st->alpha;
-  const size_t base = (size_t)blockIdx.x * BLOCK_CELLS;
-#pragma unroll 4
-  for (int m = 0; m < 16; ++m) {
-    const size_t s = base + threadIdx.x + THREADS * m;
-    z[s] = a * x[s] + y[s];
-  }
-}
-
-// BiCGSTAB update (FFVILS.h:938-958): AXPBYPZ(x, p_, s_, alpha, gamma)
-// (x = alpha*p_ + gamma*s_ + x, blas.f90:432-464), AXPYZ(r, t_, s, -gamma)
-// (r = (-gamma)*t_ + s), and r.r for IsConverged.
-__global__ void __launch_bounds__(THREADS)
-bicg_update_kernel(double* __restrict__ x, const double* __restrict__ pz,
-                   const double* __restrict__ sz, double* __restrict__ r,
-                   const double* __restrict__ t, const double* __restrict__ s,
-                   double* __restrict__ partials, SolveState* st, int iter) {
-  if (solve_done(st)) return;
-  const double alpha = st->alpha, gamma = st->gamma, mgamma = -st->gamma;
-  const size_t base = (size_t)blockIdx.x * BLOCK_CELLS;
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-#pragma unroll 4
-    for (int m = 0; m < 8; ++m) {
-      const size_t i = base + c * HALF_CELLS + threadIdx.x + THREADS * m;
-      x[i] = alpha * pz[i] + gamma * sz[i] + x[i];
-      const double rn = mgamma * t[i] + s[i];
-      r[i] = rn;
-      acc[c][m & 1] += rn * rn;
-    }
-  }
-  reduce_finalize(acc, partials, st, FIN_BI_RR, iter);
-}
-
-// x = x + alpha p; r = r + (-alpha) q (axpy, blas.f90:329-361); r.r.
-__global__ void __launch_bounds__(THREADS)
-cg_update_kernel(double* __restrict__ x, const double* __restrict__ p, double* __restrict__ r,
-                 const double* __restrict__ q, double* __restrict__ partials, SolveState* st,
-                 int iter) {
-  if (solve_done(st)) return;
-  const double alpha = st->alpha, malpha = -alpha;
-  const size_t base = (size_t)blockIdx.x * BLOCK_CELLS;
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-#pragma unroll 4
-    for (int m = 0; m < 8; ++m) {
-      const size_t s = base + c * HALF_CELLS + threadIdx.x + THREADS * m;
-      x[s] = x[s] + alpha * p[s];
-      const double rn = r[s] + malpha * q[s];
-      r[s] = rn;
-      acc[c][m & 1] += rn * rn;
-    }
-  }
-  reduce_finalize(acc, partials, st, FIN_CG_RR, iter);
-}
-
 // x.y over interior cells (dot, blas.f90:466-499) with a finaliser.
 __global__ void __launch_bounds__(THREADS)
 dot_kernel(const double* __restrict__ x, const double* __restrict__ y,
@@ -737,18 +639,6 @@ void launch_calc_r(cudaStream_t s, const KCtx& C, const double* x, const double*
                    const double* A, const double* b, double* r, SolveState* st) {
   calc_r_kernel<<<C.nb, THREADS, 0, s>>>(C, x, gst, A, b, r, st);
 }
-void launch_p_update(cudaStream_t s, const KCtx& C, const double* z, double* p, int first,
-                     SolveState* st) {
-  p_update_kernel<<<C.nb, THREADS, 0, s>>>(z, p, first, st);
-}
-void launch_bicg_p(cudaStream_t s, const KCtx& C, const double* r, double* p, const double* q,
-                   SolveState* st) {
-  bicg_p_kernel<<<C.nb, THREADS, 0, s>>>(r, p, q, st);
-}
-void launch_axpyz(cudaStream_t s, const KCtx& C, double* z, const double* x, const double* y,
-                  SolveState* st) {
-  axpyz_kernel<<<C.nb, THREADS, 0, s>>>(z, x, y, st);
-}
 void launch_sum(cudaStream_t s, const KCtx& C, const double* x, double* partials, SolveState* st,
                 int fin) {
   sum_kernel<<<C.nb, THREADS, 0, s>>>(x, partials, st, fin);
@@ -759,15 +649,6 @@ void launch_shift(cudaStream_t s, const KCtx& C, double* x, SolveState* st) {
 void launch_dot_rr0(cudaStream_t s, const KCtx& C, const double* r, double* r0, double* partials,
                     SolveState* st, int fin, int iter) {
   dot_rr0_kernel<<<C.nb, THREADS, 0, s>>>(r, r0, partials, st, fin, iter);
-}
-void launch_bicg_update(cudaStream_t s, const KCtx& C, double* x, const double* pz,
-                        const double* sz, double* r, const double* t, const double* sv,
-                        double* partials, SolveState* st, int iter) {
-  bicg_update_kernel<<<C.nb, THREADS, 0, s>>>(x, pz, sz, r, t, sv, partials, st, iter);
-}
-void launch_cg_update(cudaStream_t s, const KCtx& C, double* x, const double* p, double* r,
-                      const double* q, double* partials, SolveState* st, int iter) {
-  cg_update_kernel<<<C.nb, THREADS, 0, s>>>(x, p, r, q, partials, st, iter);
 }
 void launch_dot(cudaStream_t s, const KCtx& C, const double* x, const double* y,
                 double* partials, SolveState* st, int fin, int iter) {

@@ -265,29 +265,38 @@ MixCtx krylov_mix_ctx(const ffvgpu_pool* P, int fin) {
 // CTAs of the pipelined kernel.
 int krylov_grid(ffvgpu_pool* P) {
   if (!P->grid_mvpipe) {
-    int a, b, c, d, e;
-    mx_grid_sizes(P->m_threads, &a, &b, &c, &d, &e);
-    P->grid_mvpipe = e;
+    P->grid_mvpipe = matvec_block_grid();
   }
   return P->grid_cap > 0 && P->grid_cap < P->grid_mvpipe ? P->grid_cap : P->grid_mvpipe;
 }
 
 // q = A x and q.w (fin FIN_BI_QR0 or FIN_CG_QP), or with t.t as well
-// (FIN_BI_TS, then FIN_BI_TT) when 'two'.
+// (FIN_BI_TS, then FIN_BI_TT) when 'two'.  gin: x's pushed guides (or null).
 void krylov_matvec(ffvgpu_pool* P, const double* x, double* q, const double* w, int fin,
-                   bool two) {
-  const int grid = krylov_grid(P);
-  launch_mx_matvec(P->stream, krylov_mix_ctx(P, fin), grid, two ? 2 : 1, 0, 0, x, P->A, q, w,
-                   true);
+                   bool two, const double* gin) {
+  MixCtx C = krylov_mix_ctx(P, fin);
+  C.gin = gin;
+  launch_mx_matvec(P->stream, C, krylov_grid(P), two ? 2 : 1, 0, 0, x, P->A, q, w, true);
 }
 
-// A Jacobi sweep from a stored iterate, y = J(x; A, b), on the same kernel;
-// with dot also b.y (FIN_CG_RR1).
-void krylov_jacobi(ffvgpu_pool* P, const double* x, double* y, const double* b, double omega,
-                   bool dot) {
-  const int grid = krylov_grid(P);
-  launch_jacobi_pipe(P->stream, krylov_mix_ctx(P, dot ? FIN_CG_RR1 : 0), grid, dot, x, P->A, b,
-                     y, omega);
+// The Jacobi passes after the one from zero: z[0] holds that one's result and
+// gpush[0] its guides; returns the buffer with the last one's, whose guides are
+// in gpush[(K - 1) & 1].  With dot the last also forms b.z (FIN_CG_RR1).
+double* krylov_jacobi(ffvgpu_pool* P, double* const z[2], const double* b, int K, double omega,
+                      bool dot, int64_t& words, int64_t& coef, int& launches) {
+  for (int k = 2; k <= K; ++k) {
+    const bool last = k == K;
+    MixCtx C = krylov_mix_ctx(P, dot && last ? FIN_CG_RR1 : 0);
+    C.gin = P->gpush[k & 1];
+    // the vector after CG's last pass is not a stencil's operand (p is)
+    C.gout = dot && last ? nullptr : P->gpush[(k - 1) & 1];
+      launch_jacobi_block(P->stream, C, krylov_grid(P), dot && last, z[k & 1], P->A, b,
+                        z[(k - 1) & 1], omega);
+    words += 10;
+    coef += 7;
+    launches++;
+  }
+  return z[(K - 1) & 1];
 }
 
 // Derives the neighbour table from levels and block indices.
@@ -1075,7 +1084,7 @@ ffvgpu_status ffvgpu_solve_cg(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   std::memset(&R, 0, sizeof(R));
   if ((s = ensure_hist(P, N > 0 ? N : 1))) return s;
   if ((s = reset_state(P, prm->epsilon, N, P->hist_d))) return s;
-  if ((s = ensure_kpipe(P))) return s;
+  if ((s = ensure_kpipe(P)) || (s = ensure_push(P))) return s;
   const KCtx C = P->ctx(P->bc_p);
   const int every = prm->check_every > 0 ? prm->check_every : 16;
   const bool poll = prm->epsilon > 0.0;
@@ -1109,26 +1118,31 @@ ffvgpu_status ffvgpu_solve_cg(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   }
   CK(cudaEventRecord(P->ev2, P->stream));
   const int launches_before = launches;
-  for (c = 1; c <= N; ++c) {
-    // z = Jacobi^K(0) with b = r; last pass also forms r.z
-    launch_jacobi(P->stream, C, K == 1, P->z[0], P->A, P->r, prm->omega, P->partials, P->st);
+  if (K > 1) {
+    launch_jacobi_zero(P->stream, C, P->r, P->A, P->z[0], prm->omega, P->gpush[0], P->st);
+    launches++;
     words += 9;
     coef += 7;
-    launches++;
-    for (int k = 2; k <= K; ++k) {
-      krylov_jacobi(P, P->z[(k - 2) & 1], P->z[(k - 1) & 1], P->r, prm->omega, k == K);
-      words += 10;
+  }
+  for (c = 1; c <= N; ++c) {
+    // z = Jacobi^K(0) with b = r; the last pass also forms r.z.  The pass from
+    // zero comes with the update of r (K > 1), or is the only one
+    if (K == 1) {
+      launch_jacobi(P->stream, C, true, P->z[0], P->A, P->r, prm->omega, P->partials, P->st);
+      words += 9;
       coef += 7;
       launches++;
     }
-    const double* z = P->z[(K - 1) & 1];
-    launch_p_update(P->stream, C, z, P->p, c == 1 ? 1 : 0, P->st);
+    double* z = krylov_jacobi(P, P->z, P->r, K, prm->omega, true, words, coef, launches);
+    launch_cg_p(P->stream, C, z, P->p, P->gpush[0], P->st, c);
     words += c == 1 ? 2 : 3;
-    krylov_matvec(P, P->p, P->q, P->p, FIN_CG_QP, false);  // x, A, w, y
+    krylov_matvec(P, P->p, P->q, P->p, FIN_CG_QP, false, P->gpush[0]);  // x, A, w, y
     words += 10;
     coef += 7;
-    launch_cg_update(P->stream, C, x, P->p, P->r, P->q, P->partials, P->st, c);
-    words += 6;
+    launch_cg_update(P->stream, C, x, P->p, P->r, P->q, P->A, K > 1 ? P->z[0] : nullptr,
+                     prm->omega, P->gpush[0], P->kpart, P->st, c);
+    words += 6 + (K > 1 ? 8 : 0);
+    coef += K > 1 ? 7 : 0;
     launches += 3;
     if (poll && (c % every) == 0) {
       bool done = false;
@@ -1163,30 +1177,6 @@ ffvgpu_status ffvgpu_solve_cg(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
 }
 
 
-// Jacobi_PreConditioner (FFVILS.h:469-492) from z = 0 with right-hand side
-// rhs: K passes through the two buffers zz; returns the buffer holding the
-// result.  K = 0 leaves the zero field.
-static double* jacobi_pre(ffvgpu_pool* P, const KCtx& C, double* const zz[2], const double* rhs,
-                          int K, double omega, int64_t& words, int64_t& coef, int& launches) {
-  if (K <= 0) {
-    launch_fill(P->stream, P->nb, zz[0], BC, nullptr, 0.0);
-    words += 1;
-    launches++;
-    return zz[0];
-  }
-  launch_jacobi(P->stream, C, false, zz[0], P->A, rhs, omega, P->partials, P->st);
-  words += 9;
-  coef += 7;
-  launches++;
-  for (int k = 2; k <= K; ++k) {
-    krylov_jacobi(P, zz[(k - 2) & 1], zz[(k - 1) & 1], rhs, omega, false);
-    words += 10;
-    coef += 7;
-    launches++;
-  }
-  return zz[(K - 1) & 1];
-}
-
 // FFVILS::BiCGSTAB (src/FFV/FFVILS.h:793-974), Jacobi-preconditioned: the
 // reference's default pressure solver.  As in CG, guide cells of p and s are
 // never read by a stencil (they are right-hand sides of the preconditioner
@@ -1212,7 +1202,7 @@ ffvgpu_status ffvgpu_solve_bicgstab(ffvgpu_pool* P, const ffvgpu_iter_params* pr
   if (!(prm->restart_drop >= 0.0 && prm->restart_drop < 1.0))
     return bad("restart_drop must lie in [0, 1)");
   if ((s = reset_state(P, prm->epsilon, N, P->hist_d, prm->restart_drop))) return s;
-  if ((s = ensure_kpipe(P))) return s;
+  if ((s = ensure_kpipe(P)) || (s = ensure_push(P))) return s;
   const KCtx C = P->ctx(P->bc_p);
   const int every = prm->check_every > 0 ? prm->check_every : 16;
   const bool poll = prm->epsilon > 0.0;
@@ -1237,19 +1227,35 @@ ffvgpu_status ffvgpu_solve_bicgstab(ffvgpu_pool* P, const ffvgpu_iter_params* pr
   const int K = prm->pre_count;
   CK(cudaEventRecord(P->ev2, P->stream));
   const int launches_before = launches;
+  if (N >= 1) {
+    launch_dot_rr0(P->stream, C, P->r, P->r0, P->partials, P->st, FIN_BI_RR1, 1);  // rr1
+    launches++;
+    words += 2;
+    if (K <= 0) {  // p_ and s_ stay the zero field
+      launch_fill(P->stream, P->nb, P->z[0], BC, nullptr, 0.0);
+      launch_fill(P->stream, P->nb, P->zb[0], BC, nullptr, 0.0);
+      words += 2;
+      launches += 2;
+    }
+  }
   for (int c = 1; c <= N; ++c) {
-    launch_dot_rr0(P->stream, C, P->r, P->r0, P->partials, P->st, FIN_BI_RR1, c);  // rr1
-    launch_bicg_p(P->stream, C, P->r, P->p, P->q, P->st);
-    const double* pz = jacobi_pre(P, C, P->z, P->p, K, prm->omega, words, coef, launches);
-    krylov_matvec(P, pz, P->q, P->r0, FIN_BI_QR0, false);
-    launch_axpyz(P->stream, C, P->sv, P->q, P->r, P->st);
-    const double* sz = jacobi_pre(P, C, P->zb, P->sv, K, prm->omega, words, coef, launches);
-    krylov_matvec(P, sz, P->tv, P->sv, FIN_BI_TS, true);  // t_.s and t_.t
-    launch_bicg_update(P->stream, C, x, pz, sz, P->r, P->tv, P->sv, P->partials, P->st, c);
-    launches += 6;
-    // r.r0, p, two A*x (x, A, w, y), s, the update
-    words += 2 + (c == 1 ? 2 : 4) + 10 + 3 + 10 + 9;
-    coef += 14;
+    double* pz = P->z[0];
+    double* sz = P->zb[0];
+    launch_bicg_p(P->stream, C, P->r, P->p, P->q, P->r0, P->A, K > 0 ? P->z[0] : nullptr,
+                  prm->omega, P->gpush[0], P->st);
+    if (K > 0) pz = krylov_jacobi(P, P->z, P->p, K, prm->omega, false, words, coef, launches);
+    const double* g = K > 0 ? P->gpush[(K - 1) & 1] : nullptr;
+    krylov_matvec(P, pz, P->q, P->r0, FIN_BI_QR0, false, g);
+    launch_bicg_s(P->stream, C, P->sv, P->q, P->r, P->A, K > 0 ? P->zb[0] : nullptr, prm->omega,
+                  P->gpush[0], P->st);
+    if (K > 0) sz = krylov_jacobi(P, P->zb, P->sv, K, prm->omega, false, words, coef, launches);
+    krylov_matvec(P, sz, P->tv, P->sv, FIN_BI_TS, true, g);  // t_.s and t_.t
+    launch_bicg_update(P->stream, C, x, pz, sz, P->r, P->tv, P->sv, P->r0, P->kpart, P->st, c);
+    launches += 5;
+    // p, s (with their first Jacobi pass: z written, A read), two A*x (x, A, w,
+    // y), the update (with r0)
+    words += (c == 1 ? 3 : 4) + 3 + (K > 0 ? 16 : 0) + 20 + 8;
+    coef += 14 + (K > 0 ? 14 : 0);
     if (poll && (c % every) == 0) {
       bool done = false;
       if ((s = poll_done(P, &done))) return s;

@@ -241,12 +241,12 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* __restrict__ xin
   ok = ok && (blk < 0 || wait_rec(0));
   int n = 0;
   if (skip) blk = -1;  // the copies in flight are drained below
+  double X[2][NC];
+  Staging<SRC> L;
+  if (ok && blk >= 0) L.load(X, xin, blk, S.rec[0].nbr, gst);
   while (blk >= 0) {
     const int k = n & 1;
     const Record& R = S.rec[n % 3];
-    double X[2][NC];
-    Staging<SRC> L;
-    if (ok) L.load(X, xin, blk, R.nbr, gst);
     if (SWEEP && n > 0) __syncthreads();  // the pushes of the block before are out of the tile
     if (ok) L.put(T, X, xin, blk, R.nbr, C.bc, C.dx);
     if (tid == 0) S.next[k] = block_of(drawn);
@@ -280,6 +280,8 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* __restrict__ xin
     if (RES) warp_sums(acc, S.ws[k]);
     async::fence_proxy_async();  // b[k] is refilled by a bulk copy after the barriers
     __syncthreads();
+    // the next block's loads are in flight over the pushes
+    if (PER_SM > 1 && next >= 0) L.load(X, xin, next, S.rec[(n + 1) % 3].nbr, gst);
     if (RES && tid == 0) __stcg(partials + blk, block_sum(S.ws[k]));
     if (SWEEP && gout) push_guides(T, R.nbr, gout);
     if constexpr (PER_SM == 1)
