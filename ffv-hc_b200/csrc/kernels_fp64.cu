@@ -317,37 +317,72 @@ exchange_kernel(KCtx C, const double* __restrict__ x, double* __restrict__ g) {
 }
 
 // Host layout block (n+2vc)^3 -> colour-split interior (+ layer-1 guides).
+// 'stage' is often pinned host memory, read across the link, so the rows a
+// block needs are read whole and in the order they lie in: of each plane
+// k = 0..15 the rows j = 0..15 (with guides -1..16), and with guides the same
+// rows of planes -1 and 16 -- runs of at least 16 w doubles, V of them per load,
+// every load in flight before the first store.  The link moves 32-byte
+// sectors, so a row's 16 interior values, 16 bytes into it, cost all of its 160
+// (vc = 2) anyway.  They go through shared memory to their places.
+// 1164 blocks, vc = 2, pinned: with guides 1837 -> 1285 us (59.6 MB, 46 GB/s; read
+// value by value, the x-face guides cost a sector each), without 954 -> 965 us
+// (47.7 MB, 49 GB/s).
+template <int V>
 __global__ void __launch_bounds__(THREADS)
 pack_kernel(const double* __restrict__ stage, int vc, double* __restrict__ dst, size_t stride,
             double* __restrict__ gdst) {
+  extern __shared__ __align__(16) double rows[];
   const int blk = blockIdx.x, tid = threadIdx.x;
-  const int w = 16 + 2 * vc;
+  const int w = 16 + 2 * vc, g = gdst ? 1 : 0;
   const double* sb = stage + (size_t)blk * w * w * w;
-  // the interior row by row (16 threads read one row of 16 consecutive
-  // values: whole sectors, also when 'stage' is pinned host memory read
-  // across the link), every load in flight before the colour-split stores
-  const int i = tid & 15, r0 = tid >> 4;
-  double v[16];
+  // run p of the block: plane k = p (p < 16), then planes -1 and 16; rows[] holds
+  // them back to back, planes 0..15 with 16 + 2 g rows each
+  const int len = (16 + 2 * g) * w, total = 16 * len + g * 2 * 16 * w;
+  constexpr int U = V == 2 ? 8 : 16;
+  for (int e0 = tid * V; e0 < total; e0 += THREADS * V * U) {
+    double v[U][V];
 #pragma unroll
-  for (int m = 0; m < 16; ++m) {
-    const int r = r0 + 16 * m, j = r & 15, k = r >> 4;
-    v[m] = sb[(i + vc) + w * ((j + vc) + w * (k + vc))];
-  }
-#pragma unroll
-  for (int m = 0; m < 16; ++m) {
-    const int r = r0 + 16 * m, j = r & 15, k = r >> 4;
-    dst[(size_t)blk * stride + ((i + j + k) & 1) * HALF_CELLS + (k * 16 + j) * 8 + (i >> 1)] = v[m];
-  }
-  if (gdst) {
-    const int a = tid & 15, b = tid >> 4;
-    for (int f = 0; f < 6; ++f) {
-      int g[3];
-      const int axis = f >> 1;
-      if (axis == 0) { g[1] = a; g[2] = b; } else if (axis == 1) { g[0] = a; g[2] = b; } else { g[0] = a; g[1] = b; }
-      g[axis] = (f & 1) ? 16 : -1;
-      gdst[((size_t)blk * 6 + f) * FACE_CELLS + b * 16 + a] =
-          sb[(g[0] + vc) + w * ((g[1] + vc) + w * (g[2] + vc))];
+    for (int u = 0; u < U; ++u) {
+      const int e = e0 + u * THREADS * V;
+      if (e >= total) continue;
+      const bool side = e >= 16 * len;
+      const int f = side ? e - 16 * len : e;
+      const int p = side ? f / (16 * w) : f / len;
+      const int k = side ? (p ? 16 : -1) : p, j0 = side ? 0 : -g;
+      const double* src = sb + (size_t)((k + vc) * w + (j0 + vc)) * w + (f - p * (side ? 16 * w : len));
+      if (V == 2) {
+        const double2 t = *reinterpret_cast<const double2*>(src);
+        v[u][0] = t.x;
+        v[u][V - 1] = t.y;
+      } else {
+        v[u][0] = *src;
+      }
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = e0 + u * THREADS * V;
+      if (e >= total) continue;
+#pragma unroll
+      for (int h = 0; h < V; ++h) rows[e + h] = v[u][h];
+    }
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int m = 0; m < 16; ++m) {
+    const int s = tid + THREADS * m;
+    int i, j, k;
+    cell_of(s, i, j, k);
+    dst[(size_t)blk * stride + s] = rows[k * len + (j + g) * w + i + vc];
+  }
+  if (!gdst) return;
+  const int a = tid & 15, b = tid >> 4;
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const int out = (f & 1) ? 16 : -1;
+    const int at = f < 2   ? b * len + (a + 1) * w + out + vc
+                   : f < 4 ? b * len + (out + 1) * w + a + vc
+                           : 16 * len + (f & 1) * 16 * w + b * w + a + vc;
+    gdst[((size_t)blk * 6 + f) * FACE_CELLS + tid] = rows[at];
   }
 }
 
@@ -659,7 +694,12 @@ void launch_exchange(cudaStream_t s, const KCtx& C, const double* x, double* g) 
 }
 void launch_pack(cudaStream_t s, int nb, const double* stage, int vc, double* dst, size_t stride,
                  double* gdst) {
-  pack_kernel<<<nb, THREADS, 0, s>>>(stage, vc, dst, stride, gdst);
+  const int w = 16 + 2 * vc, rows = gdst ? 16 * 18 + 32 : 16 * 16;
+  // runs start at multiples of w (even) doubles, so pairs are aligned where the buffer is
+  auto kernel = reinterpret_cast<uintptr_t>(stage) % 16 == 0 ? pack_kernel<2> : pack_kernel<1>;
+  const int bytes = rows * w * (int)sizeof(double);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  kernel<<<nb, THREADS, bytes, s>>>(stage, vc, dst, stride, gdst);
 }
 void launch_pack_flag(cudaStream_t s, int nb, const int32_t* stage, int vc, uint8_t* flags,
                       int bit, int mode) {
