@@ -27,25 +27,24 @@ struct MixCtx {
   int capacity;
   int first;
   uint64_t wait_ns;    // limit of every bounded device wait (ffvgpu_pool_set_wait_limit)
-  int stall;           // test hook: 1 the sweep kernel, 2 the A*x of form 0 issues no copy,
+  int stall;           // test hook: 1 the sweep kernel, 2 the pipelined A*x issues no copy,
                        // so its first wait runs out
   int cf;              // coarse-fine flux correction in the FP64 residual and A*x
   int depth;           // sweep kernel: L2 prefetch distance in blocks (staging depth, >= 1)
   int sweep_threads;   // sweep kernel: 256 (two rows per thread, the default) or 512 (one row)
-  // A*x of form 0 only: 0 the mixed form's finalisers, else the FP64
-  // solver's (one instance): FIN_BI_QR0 or FIN_CG_QP on the one sum, or
-  // FIN_BI_TS on the first of two sums and FIN_BI_TT on the second
-  int fin = 0;
-  // A*x and Jacobi pass (matvec_block.cu): guides pushed by the kernel that
-  // made x (null: taken from the neighbours' interiors), and where a Jacobi
+  // the FP64 solvers' A*x and Jacobi passes (matvec_block.cu, one instance):
+  // finaliser FIN_BI_QR0 or FIN_CG_QP on the one sum, FIN_BI_TS on the first of
+  // two and FIN_BI_TT on the second, or FIN_CG_RR1; guides pushed by the kernel
+  // that made x (null: taken from the neighbours' interiors), and where a Jacobi
   // pass pushes those of its result
+  int fin = 0;
   const double* gin = nullptr;
   double* gout = nullptr;
 };
 
 // CTAs of the persistent grids: SMs x resident CTAs per SM of each kernel,
 // with 'threads' (128, 256 or 512) per CTA of the A*x (form 1) and update
-// kernels; mvpipe: the A*x of form 0 (matvec_block.cu, two CTAs per SM).
+// kernels; mvpipe: the pipelined A*x (one CTA per SM).
 void mx_grid_sizes(int threads, int* sweep, int* matvec, int* update, int* guides, int* mvpipe);
 // Sweep coefficients of blocks [first, first + count), MIXED_COEF_WORDS per
 // block, in the thread order of a sweep kernel of sweep_threads threads:
@@ -76,16 +75,16 @@ void launch_mx_guides(cudaStream_t s, const MixCtx& C, int count, const void* e,
 // not depend on the order (every sum runs over blocks in block order).
 void launch_mx_order_active(cudaStream_t s, const int32_t* raw, const double* ucoef,
                             int32_t* act);
-// y = A x with its dot products; form 0: matvec_block.cu ('count' CTAs,
-// two per SM), form 1: a block per CTA of 'threads' threads (C.fin 0 only).
+// y = A x with its dot products; form 0: the pipelined kernel ('count' CTAs,
+// one per SM), form 1: a block per CTA of 'threads' threads (C.fin 0 only).
 void launch_mx_matvec(cudaStream_t s, const MixCtx& C, int count, int ndot, int threads, int form,
                       const void* x, const double* A, double* y, const double* w0, bool d64);
-// The same, form 0 (matvec_block.cu), and its persistent grid.
-void launch_matvec_block(cudaStream_t s, const MixCtx& C, int count, int ndot, const void* x,
-                         const double* A, double* y, const double* w0, bool d64);
+// The FP64 solvers' y = A x with y.w0 (ndot 1) or y.w0 and y.y (2), and a Jacobi
+// sweep y = J(x; A, b) (bils.f90:5-55), with dot also b.y (matvec_block.cu):
+// 'count' CTAs of matvec_block_grid.
+void launch_matvec_block(cudaStream_t s, const MixCtx& C, int count, int ndot, const double* x,
+                         const double* A, double* y, const double* w0);
 int matvec_block_grid();
-// An FP64 Jacobi sweep y = J(x; A, b) (bils.f90:5-55) on the same kernel, with b
-// in the dot partner's place; with dot also b.y, finalised by C.fin (FIN_CG_RR1).
 void launch_jacobi_block(cudaStream_t s, const MixCtx& C, int count, bool dot, const double* x,
                          const double* A, const double* b, double* y, double omega);
 // Coarse-fine flux mismatch per face cell of the (block, face) pairs

@@ -867,6 +867,383 @@ mx_matvec_kernel(MixCtx C, const ET* __restrict__ x, const double* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
+// The same A*x and dot products as a persistent, warp-specialised kernel:
+// one CTA of 800 threads per SM walks its live blocks.
+//   producer (thread 0): through a ring of three 32 KB slots, by bulk copies,
+//     the dot partner w0 (a uniform block: all of it in one slot) or, for a
+//     block that streams its coefficients, eight slots of 512 cells with the
+//     seven coefficient rows and w0.
+//   gatherers (8 warps): a block ahead, its x widened to FP64 and its guide
+//     layer by the exchange rules, written into a padded tile: per colour
+//     [k + 1][j + 1][i >> 1] with rows of 8 values (k, j in -1..16), so every
+//     neighbour of a cell is at a fixed offset but the x-face guides, which
+//     sit in two arrays of their own; with rows of 8 the two rows a half-warp
+//     reads fall into disjoint banks.  The loads are issued before the tile
+//     frees up.
+//   consumers (16 warps): consumer t takes cells q = 512 mm + t of each
+//     colour, which makes it the block tree's virtual thread t: the per-block
+//     sums are those of mx_reduce; the ticket of an instance is advanced once
+//     per run of its blocks in the CTA's list, and the CTA that completes it
+//     forms the cross-block sums (256 lanes, block order) and finalises.
+// Every wait is bounded (MixCtx::wait_ns); a wait that gives up stops the
+// instances of the CTA's list with TIMEOUT.
+// (The FP64 solvers' A*x, matvec_block.cu, holds two smaller CTAs per SM; this
+// form suits the mixed one, whose FP32 x has no pushed guides: a batch of 16
+// instances, 5695 blocks, 24 iterations 45.1 ms against 46.3.)
+// ---------------------------------------------------------------------------
+namespace mvp {
+constexpr int STAGES = 3;
+constexpr int ROWS = 8;                            // A rows 0..6 (Ap, Aw..At), w0
+constexpr int SLOT_CELLS = 512;
+constexpr int SLOTS = BLOCK_CELLS / SLOT_CELLS;    // slots of a streamed block
+constexpr uint32_t SLOT_BYTES = ROWS * SLOT_CELLS * 8;
+constexpr int GATHER0 = 32, NGATHER = 256;
+constexpr int CONS0 = GATHER0 + NGATHER, NCONS = 512, CONS_WARPS = NCONS / 32;
+constexpr int NTHREADS = CONS0 + NCONS;            // 800
+constexpr int CAP = NTHREADS;                      // list entries per chunk
+constexpr int ROLE_MATVEC = 32;                    // SolveState::timeout_where bit
+static_assert(SLOT_BYTES == BLOCK_CELLS * 8, "a slot holds a uniform block's w0");
+// the tile: row pitch (i >> 1 in 0..7), plane pitch (rows j = -1..16) and
+// colour half (planes k = -1..16)
+constexpr int TR = 8, TP = 18 * TR, TH = 18 * TP, TT = 2 * TH;
+
+struct __align__(128) Smem {
+  double ring[STAGES][ROWS][SLOT_CELLS];  // 96 KB
+  double tile[2][TT];                     // 81 KB: x of the current / next block, j/k guides
+  double xg[2][2][FACE_CELLS];            // 8 KB: their x-face guides [face][j + 16 k]
+  double urec[2][8];                      // coefficient records of the blocks in the tiles
+  // warp sums of the block tree [block parity][sum][warp]: consumer 0 reads
+  // block n's while the other warps may already write block n + 1's
+  double ws[2][2][CONS_WARPS];
+  int2 list[CAP];                         // the chunk's live entries
+  FaceNbr snb[2][6];                      // face records (flux correction)
+  // full/empty: ring slots; gfull: a tile ready; tempty: a tile free
+  uint64_t full[STAGES], empty[STAGES], gfull[2], tempty[2];
+  int wcount[NTHREADS / 32];
+  int nlist, next_from, abort_flag, last_inst;
+};
+static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of one CTA");
+
+// Tile position of the j/k-face guide at (face, p = u + 16 v), face 2..5.
+__device__ __forceinline__ int tile_guide(int face, int p) {
+  const int u = p & 15, v = p >> 4, out = (face & 1) ? 16 : -1;
+  return face < 4 ? ((u + out + v) & 1) * TH + (v + 1) * TP + (out + 1) * TR + (u >> 1)
+                  : ((u + v + out) & 1) * TH + (out + 1) * TP + (v + 1) * TR + (u >> 1);
+}
+// The first guide layer of a tile read as [face][p] (flux correction).
+struct TileGuides {
+  const double* T;
+  const double* XG;  // [2][256]
+  __device__ double operator[](int g) const {
+    const int f = g >> 8, p = g & 255;
+    return f < 2 ? XG[f * FACE_CELLS + p] : T[tile_guide(f, p)];
+  }
+};
+
+__device__ __forceinline__ void consumer_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(NCONS) : "memory");
+}
+__device__ __forceinline__ void release_slot(uint64_t* bar, int lane, bool live) {
+  async::fence_proxy_async();
+  __syncwarp();
+  if (lane == 0 && live) async::mbar_arrive(bar);
+}
+}  // namespace mvp
+
+template <int NV, bool CF, typename ET>
+__global__ void __launch_bounds__(mvp::NTHREADS, 1)
+mx_matvec_pipe_kernel(MixCtx C, const ET* __restrict__ x, const double* __restrict__ A,
+                      double* __restrict__ y, const double* __restrict__ w0) {
+  using namespace mvp;
+  static_assert(NV == 1 || NV == 2, "sums of the kernel");
+  using async::mbar_wait;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  Smem& S = *reinterpret_cast<Smem*>(smem_raw);
+  const int tid = threadIdx.x;
+  volatile int* abort_flag = &S.abort_flag;
+  const int n_act = *C.n_active;
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      async::mbar_init(&S.full[s], 1);
+      async::mbar_init(&S.empty[s], CONS_WARPS);
+    }
+    for (int b = 0; b < 2; ++b) {
+      async::mbar_init(&S.gfull[b], NGATHER);
+      async::mbar_init(&S.tempty[b], 1);
+    }
+    S.abort_flag = 0;
+    async::fence_mbar_init();
+  }
+  // Counters that run across the chunks: ring slots issued (producer) or
+  // consumed (consumers), blocks of earlier chunks.
+  uint32_t g = 0;
+  int M0 = 0;
+  int run = 0;  // consumer 0: blocks of the current instance not yet on its ticket
+  bool live = true;
+  for (int from = blockIdx.x; from < n_act;) {
+    build_live_list<1, false, NTHREADS, CAP>(C, from, n_act, S.list, &S.nlist, &S.next_from,
+                                             S.wcount);
+    from = S.next_from;
+    const int nl = S.nlist;
+    auto is_uni = [&](int n) { return (S.list[n].y & LF_UNI) != 0; };
+    if (tid == 0 && nl > 0 && !*abort_flag) {
+      // ------------------------------------------------------------ producer
+      // (test hook MixCtx::stall == 2: no copy is issued, so the consumers'
+      // first wait for a slot runs out)
+      for (int n = 0; n < nl && C.stall != 2; ++n) {
+        const size_t blk = (size_t)S.list[n].x;
+        const int ns = is_uni(n) ? 1 : SLOTS;
+        bool ok = true;
+        for (int j = 0; j < ns; ++j, ++g) {
+          const int s = g % STAGES;
+          if (!(ok = mbar_wait(&S.empty[s], ((g / STAGES) & 1) ^ 1, abort_flag, ROLE_MATVEC,
+                               C.wait_ns)))
+            break;
+          async::mbar_expect_tx(&S.full[s], SLOT_BYTES);
+          if (ns == 1) {
+            async::bulk_g2s(S.ring[s], w0 + blk * BLOCK_CELLS, SLOT_BYTES, &S.full[s]);
+          } else {
+#pragma unroll 1
+            for (int a = 0; a < 7; ++a)
+              async::bulk_g2s(S.ring[s][a], A + (blk * 7 + a) * BLOCK_CELLS + j * SLOT_CELLS,
+                              SLOT_CELLS * 8, &S.full[s]);
+            async::bulk_g2s(S.ring[s][7], w0 + blk * BLOCK_CELLS + j * SLOT_CELLS,
+                            SLOT_CELLS * 8, &S.full[s]);
+          }
+        }
+        if (!ok) break;
+      }
+    } else if (tid >= GATHER0 && tid < CONS0) {
+      // ----------------------------------------------------------- gatherers
+      const int gt = tid - GATHER0, grp = gt >> 7, p0 = gt & 127, p1 = p0 + 128;
+      for (int n = 0; n < nl; ++n) {
+        const int Mg = M0 + n, b = Mg & 1;
+        const int blk = S.list[n].x;
+        const double dx = C.dx[blk];
+        // everything this thread writes into the tile, loaded before the tile
+        // (block Mg - 2) is free: 16 values of x (cells gt + 256 m: a
+        // half-warp's stores then fill 16 consecutive tile positions, one
+        // bank each), and two positions of alternate faces of the guide layer
+        ET xv[16];
+        const ET* xb = x + (size_t)blk * BLOCK_CELLS;
+#pragma unroll
+        for (int m = 0; m < 16; ++m) xv[m] = __ldg(xb + gt + NGATHER * m);
+        double gv[3][2];
+        FaceNbr nfs[CF ? 3 : 1];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          const int f = 2 * r + grp;
+          const FaceNbr nf = C.nbr[blk * 6 + f];
+          guide_pair(x, blk, f, p0, p1, nf, C.bc, dx, gv[r][0], gv[r][1]);
+          if (CF) nfs[CF ? r : 0] = nf;
+        }
+        const double ur = gt < 8 ? __ldg(C.ucoef + (size_t)blk * 8 + gt) : 0.0;
+        if (Mg >= 2 &&
+            !mbar_wait(&S.tempty[b], ((Mg - 2) >> 1) & 1, abort_flag, ROLE_MATVEC, C.wait_ns))
+          break;
+        double* T = S.tile[b];
+#pragma unroll
+        for (int m = 0; m < 16; ++m) {
+          const int s0 = gt + NGATHER * m;
+          const int c = s0 >> 11, q = s0 & 2047;
+          const int ih = q & 7, j = (q >> 3) & 15, k = q >> 7;
+          T[c * TH + (k + 1) * TP + (j + 1) * TR + ih] = (double)xv[m];
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          const int f = 2 * r + grp;
+          if (f < 2) {
+            S.xg[b][f][p0] = gv[r][0];
+            S.xg[b][f][p1] = gv[r][1];
+          } else {
+            T[tile_guide(f, p0)] = gv[r][0];
+            T[tile_guide(f, p1)] = gv[r][1];
+          }
+          if (CF && p0 == 0) S.snb[b][f] = nfs[CF ? r : 0];
+        }
+        if (gt < 8) S.urec[b][gt] = ur;
+        async::mbar_arrive(&S.gfull[b]);
+      }
+    } else if (tid >= CONS0) {
+      // ----------------------------------------------------------- consumers
+      // Every consumer runs the same sequence of named barriers and shuffles;
+      // only the work is predicated on 'live'.
+      const int ct = tid - CONS0, lane = ct & 31, warp = ct >> 5;
+      // this thread's cells q = 512 mm + ct: (2 ih + p, j, k0 + 4 mm), where
+      // the parity p of the row is the same for every mm
+      const int ih = ct & 7, jr = (ct >> 3) & 15, k0 = ct >> 7;
+      const int pos0 = (k0 + 1) * TP + (jr + 1) * TR + ih;  // tile position, mm = 0
+      for (int n = 0; n < nl; ++n) {
+        const int Mg = M0 + n, b = Mg & 1;
+        const uint32_t par = (Mg >> 1) & 1;
+        const int2 ent = S.list[n];
+        const int blk = ent.x, inst = ent.y & LF_INST;
+        const bool uni = ent.y & LF_UNI;
+        live = live && mbar_wait(&S.gfull[b], par, abort_flag, ROLE_MATVEC, C.wait_ns);
+        const double* T = S.tile[b];
+        const double* XG = &S.xg[b][0][0];
+        double u[7];
+#pragma unroll
+        for (int a = 0; a < 7; ++a) u[a] = uni ? S.urec[b][a] : 0.0;
+        const int us = g % STAGES;
+        if (uni)
+          live = live && mbar_wait(&S.full[us], (g / STAGES) & 1, abort_flag, ROLE_MATVEC,
+                                   C.wait_ns);
+        const double* wflat = &S.ring[us][0][0];
+        const size_t base = (size_t)blk * BLOCK_CELLS;
+        double acc[NV][2] = {};
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int p = (jr + k0 + c) & 1;
+          const double* own = T + c * TH + pos0;         // the cell
+          const double* oth = T + (1 - c) * TH + pos0;   // its position in the other colour
+          // the x-face guides take the place of the west (i = 0) and east
+          // (i = 15) neighbours
+          const bool gw = ih == 0 && p == 0, ge = ih == 7 && p == 1;
+#pragma unroll 2
+          for (int mm = 0; mm < SLOTS / 2; ++mm) {
+            const int q = mm * NCONS + ct, s = c * HALF_CELLS + q, o = mm * 4 * TP;
+            const int gq = jr + 16 * (k0 + 4 * mm);  // the x-face guides' position
+            double k[7], wv = 0.0;
+            if (uni) {
+#pragma unroll
+              for (int a = 0; a < 7; ++a) k[a] = u[a];
+              if (live) wv = wflat[s];
+            } else {
+              const int sl = g % STAGES;
+              live = live && mbar_wait(&S.full[sl], (g / STAGES) & 1, abort_flag, ROLE_MATVEC,
+                                       C.wait_ns);
+#pragma unroll
+              for (int a = 0; a < 7; ++a) k[a] = live ? S.ring[sl][a][ct] : 0.0;
+              if (live) wv = S.ring[sl][7][ct];
+              asm volatile("" ::"d"(k[0]), "d"(k[1]), "d"(k[2]), "d"(k[3]), "d"(k[4]), "d"(k[5]),
+                           "d"(k[6]), "d"(wv));
+              release_slot(&S.empty[sl], lane, live);
+              ++g;
+            }
+            if (!live) continue;
+            // neighbours w, e (i -+ 1: other colour, columns ih + p - 1 and
+            // ih + p of it), s, n (rows -+ 1), b, t (planes -+ 1); the j and k
+            // guides sit in the tile's border rows and planes
+            const double xw = gw ? XG[gq] : oth[o - 1 + p];
+            const double xe = ge ? XG[FACE_CELLS + gq] : oth[o + p];
+            const double xs = oth[o - TR], xn = oth[o + TR];
+            const double xb = oth[o - TP], xt = oth[o + TP];
+            const double xp = own[o];
+            double yv = k[1] * xw + k[2] * xe + k[3] * xs + k[4] * xn + k[5] * xb + k[6] * xt +
+                 k[0] * xp;
+            if (CF)  // coarse-fine flux correction: y = A x + delta
+              yv = cf_delta<false>(x, (const double*)nullptr, A, C.nbr, C.dx, C.bc, S.snb[b],
+                                   TileGuides{T, XG}, xp, s, yv,
+                                   [&](int f) { return k[1 + f]; });
+            y[base + s] = yv;
+            acc[0][c] += yv * wv;
+            if (NV == 2) acc[NV - 1][c] += yv * yv;
+          }
+        }
+        if (uni) {  // w0 is in registers (the loads completed before its use)
+          release_slot(&S.empty[us], lane, live);
+          ++g;
+        }
+        // block tree (mx_reduce with 512 threads): warp butterflies, then the
+        // 16 warp sums in order
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          double t = acc[v][0] + acc[v][1];
+#pragma unroll
+          for (int off = 16; off >= 1; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+          if (lane == 0) S.ws[b][v][warp] = t;
+        }
+        consumer_sync();  // every consumer is done with tile b
+        if (ct == 0 && live) {
+          async::mbar_arrive(&S.tempty[b]);
+#pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            double sum = 0.0;
+#pragma unroll
+            for (int w = 0; w < CONS_WARPS; ++w) sum += S.ws[b][v][w];
+            __stcg(C.partials + (size_t)v * C.capacity + blk, sum);
+          }
+          ++run;
+        }
+        // the instance's ticket, once per run of its blocks in this chunk
+        if (n + 1 == nl || (S.list[n + 1].y & LF_INST) != inst) {
+          if (ct == 0) {
+            int li = -1;
+            if (live && run > 0) {
+              __threadfence();
+              const unsigned t = atomicAdd(&C.inst.st[inst].ticket, (unsigned)run);
+              if (t + (unsigned)run == (unsigned)C.inst.count[inst]) li = inst;
+            }
+            run = 0;
+            S.last_inst = li;
+          }
+          consumer_sync();
+          const int li = S.last_inst;
+          if (li >= 0) {
+            // cross-block sums over the instance's blocks: lanes 0..255, block
+            // order, butterfly, 8 warp sums in order
+            __threadfence();
+            const int first = C.inst.first[li], cnt = C.inst.count[li];
+            double tot[NV];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+              double sv = 0.0;
+              if (ct < 256)
+                for (int bb = ct; bb < cnt; bb += 256)
+                  sv += __ldcg(C.partials + (size_t)v * C.capacity + first + bb);
+#pragma unroll
+              for (int off = 16; off >= 1; off >>= 1) sv += __shfl_xor_sync(0xffffffffu, sv, off);
+              consumer_sync();
+              if (lane == 0 && ct < 256) S.ws[b][0][ct >> 5] = sv;
+              consumer_sync();
+              double total = 0.0;
+#pragma unroll
+              for (int w = 0; w < 8; ++w) total += S.ws[b][0][w];
+              tot[v] = total;
+            }
+            if (ct == 0) {
+              SolveState* St = C.inst.st + li;
+              mx_finalize(St, tot, NV == 1 ? FIN_MX_ALPHA : FIN_MX_GAMMA);
+              St->ticket = 0;
+              __threadfence();
+            }
+            consumer_sync();  // S.ws is rewritten by the next block
+          }
+        }
+      }
+    }
+    M0 += nl;
+    __syncthreads();  // every role is past the chunk before its list is rebuilt
+    if (*abort_flag) break;
+  }
+  if (tid == 0) {
+    // Drain: the last armed phase of every ring slot must complete before the
+    // CTA may exit (each has at most one copy phase in flight: a slot is
+    // refilled only after its copy landed and was used).
+    bool drained = true;
+    for (int s = 0; s < STAGES; ++s) {
+      const uint32_t issued = (g > (uint32_t)s) ? (g - 1 - s) / STAGES + 1 : 0;
+      if (issued) drained = async::mbar_drain(&S.full[s], (issued - 1) & 1) && drained;
+    }
+    if (*abort_flag) {
+      // stop every instance of this CTA's chunk and of its later candidates
+      const int where = *abort_flag | (drained ? 0 : async::ROLE_DRAIN);
+      auto stop = [&](int i2) {
+        atomicOr(&C.inst.st[i2].timeout_where, where);
+        atomicExch(&C.inst.st[i2].status, 3);
+        atomicExch(&C.inst.st[i2].done, 1);
+      };
+      for (int k = 0; k < S.nlist; ++k) stop(S.list[k].y & LF_INST);
+      for (int it2 = S.next_from; it2 < n_act; it2 += gridDim.x) {
+        const int i2 = C.inst.blk_inst[C.active[it2]];
+        if (i2 >= 0) stop(i2);
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // x = alpha*p_ + gamma*s_ + x (axpbypz, blas.f90:431-464, FFVILS.h:938-944);
 // r = (-gamma)*t_ + s (axpyz, blas.f90:397-429, FFVILS.h:945-950); r.r and
 // the next iteration's r.r0.
@@ -1048,7 +1425,16 @@ void mx_grid_sizes(int threads, int* sweep, int* matvec, int* update, int* guide
   *guides = sms * std::max(1, g);
   *matvec = sms * std::max(1, c);
   *update = sms * std::max(1, d);
-  *mvpipe = matvec_block_grid();
+  // the pipelined A*x: its shared memory on this device, one CTA per SM
+#define MV_ALLOW(NV, CF, ET)                                                           \
+  cudaFuncSetAttribute(mx_matvec_pipe_kernel<NV, CF, ET>,                               \
+                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(mvp::Smem));
+  MV_ALLOW(1, false, float) MV_ALLOW(2, false, float)
+  MV_ALLOW(1, true, float) MV_ALLOW(2, true, float)
+  MV_ALLOW(1, false, double) MV_ALLOW(2, false, double)
+  MV_ALLOW(1, true, double) MV_ALLOW(2, true, double)
+#undef MV_ALLOW
+  *mvpipe = sms;
 }
 
 template <typename ET, int NT>
@@ -1129,10 +1515,26 @@ void launch_mx_order_active(cudaStream_t s, const int32_t* raw, const double* uc
   mx_order_active_kernel<<<1, 1024, 0, s>>>(raw, ucoef, act);
 }
 
+template <typename ET>
+static void matvec_pipe(cudaStream_t s, const MixCtx& C, int count, int ndot, const ET* x,
+                        const double* A, double* y, const double* w0) {
+  constexpr int T = mvp::NTHREADS, B = (int)sizeof(mvp::Smem);
+  if (ndot == 1 && !C.cf)
+    mx_matvec_pipe_kernel<1, false, ET><<<count, T, B, s>>>(C, x, A, y, w0);
+  else if (!C.cf)
+    mx_matvec_pipe_kernel<2, false, ET><<<count, T, B, s>>>(C, x, A, y, w0);
+  else if (ndot == 1)
+    mx_matvec_pipe_kernel<1, true, ET><<<count, T, B, s>>>(C, x, A, y, w0);
+  else
+    mx_matvec_pipe_kernel<2, true, ET><<<count, T, B, s>>>(C, x, A, y, w0);
+}
+
 void launch_mx_matvec(cudaStream_t s, const MixCtx& C, int count, int ndot, int threads, int form,
                       const void* x, const double* A, double* y, const double* w0, bool d64) {
-  if (form == 0)
-    launch_matvec_block(s, C, count, ndot, x, A, y, w0, d64);
+  if (form == 0 && d64)
+    matvec_pipe(s, C, count, ndot, static_cast<const double*>(x), A, y, w0);
+  else if (form == 0)
+    matvec_pipe(s, C, count, ndot, static_cast<const float*>(x), A, y, w0);
   else if (d64)
     matvec_nt(s, C, count, ndot, threads, static_cast<const double*>(x), A, y, w0);
   else

@@ -1,6 +1,6 @@
 // matvec_block.cu -- A x with its dot products, and a Jacobi pass, for sm_100a:
 // the stencil kernels of the FP64 Krylov solvers (FFVILS::CG and BiCGSTAB,
-// src/FFV/FFVILS.h:661-974) and of the mixed form.
+// src/FFV/FFVILS.h:661-974).
 //
 // y = A x (calc_ax, src/CGMfuncs/bils.f90:162-206) with y.w0 (NV 1: q_.r0 or
 // q.p) or y.w0 and y.y (NV 2: t_.s and t_.t_); or, JAC, a Jacobi sweep of x with
@@ -15,7 +15,7 @@
 // leaves.  Level-5 sphere grid, us per launch, one 800-thread warp-specialised
 // CTA per SM before -> here: A x with q.r0 154 -> 123, with t.s and t.t
 // 164 -> 128, a Jacobi pass 152 -> 140 (87 us at the measured 6463 GB/s for the
-// 561 MB that must move); FP32 x: 140 / 151 -> 133 / 138.  Tried without gain:
+// 561 MB that must move).  Tried without gain:
 // w0 in registers (more L1, but spills), three CTAs' worth of carve-out.
 #include <algorithm>
 #include <cstddef>
@@ -83,10 +83,10 @@ __device__ __forceinline__ void divide(const Rows&, double (&rs)[N], const doubl
 // The cells of one staged block; w and y start at the thread's first cell.
 // With JAC the new values replace X (a cell's neighbours are of the other
 // colour: colour 0 is formed into Y first).
-template <int NV, bool JAC, typename COEF, typename CFF>
+template <int NV, bool JAC, typename COEF>
 __device__ __forceinline__ void cells(const double* T, double (&X)[2][NC], const COEF& A,
                                       const double* w, double* __restrict__ y, double omega,
-                                      double (&acc)[2][2][2], const CFF& cf) {
+                                      double (&acc)[2][2][2]) {
   constexpr int G = 4;  // cells whose loads are in flight together
   double Y0[JAC ? NC : 1];
 #pragma unroll
@@ -107,7 +107,6 @@ __device__ __forceinline__ void cells(const double* T, double (&X)[2][NC], const
         } else {
           v[n - n0] = k.w * b.w + k.e * b.e + k.s * b.s + k.n * b.n + k.b * b.b + k.t * b.t +
                       k.p * X[c][n];
-          v[n - n0] = cf(s, X[c][n], v[n - n0], k);
         }
       }
       if (JAC) {
@@ -135,12 +134,11 @@ __device__ __forceinline__ void cells(const double* T, double (&X)[2][NC], const
     for (int n = 0; n < NC; ++n) X[0][n] = Y0[JAC ? n : 0];
 }
 
-template <int NV, bool CF, typename ET, bool JAC, int SRC>
+template <int NV, bool JAC, int SRC>
 __global__ void __launch_bounds__(NT, 2)
-matvec_block_kernel(const __grid_constant__ MixCtx C, const ET* __restrict__ x,
+matvec_block_kernel(const __grid_constant__ MixCtx C, const double* __restrict__ x,
                     const double* __restrict__ A, double* __restrict__ y,
                     const double* __restrict__ w0, double omega) {
-  static_assert(!(JAC && CF), "the Jacobi sweep has no flux correction");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Smem& S = *reinterpret_cast<Smem*>(smem_raw);
   double* T = S.tile;
@@ -153,14 +151,12 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const ET* __restrict__ x,
   }
   __syncthreads();
   const int n_act = *C.n_active;
-  // test hook (MixCtx::stall == 2): nothing is fetched, so the first wait runs out
-  const bool fetch = C.stall != 2;
   auto fetch_rec = [&](int blk, int m) {  // record of the CTA's m-th block
-    if (fetch && tid < REC_THREADS)
+    if (tid < REC_THREADS)
       fetch_record(S.rec[m % 3], &S.rbar[m % 3], C.nbr, C.ucoef, blk);
   };
   auto fetch_w = [&](int blk, int m) {  // w0 of the CTA's m-th block
-    if (fetch && tid == 32) {
+    if (tid == 32) {
       async::mbar_expect_tx(&S.wbar[m & 1], BLOCK_CELLS * 8);
       async::bulk_g2s(S.w[m & 1], w0 + (size_t)blk * BLOCK_CELLS, BLOCK_CELLS * 8, &S.wbar[m & 1]);
     }
@@ -205,7 +201,7 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const ET* __restrict__ x,
       if (next >= 0) {
         fetch_w(next, n + 1);
         if (tid == 64)
-          async::prefetch_l2(x + (size_t)next * BLOCK_CELLS, BLOCK_CELLS * (uint32_t)sizeof(ET));
+          async::prefetch_l2(x + (size_t)next * BLOCK_CELLS, BLOCK_CELLS * 8);
         if (tid == 96 && S.rec[(n + 1) % 3].u[7] == 0.0)
           async::prefetch_l2(A + (size_t)next * 7 * BLOCK_CELLS, 7 * BLOCK_CELLS * 8);
       }
@@ -213,18 +209,10 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const ET* __restrict__ x,
       const double* w = S.w[k] + slot(tid);
       double* yb = y + (size_t)blk * BLOCK_CELLS + slot(tid);
       double acc[2][2][2] = {};
-      auto cf = [&](int s, double xp, double v, const K7& a) {
-        if (!CF) return v;  // coarse-fine flux correction: y = A x + delta
-        return cf_delta<false>(x, (const double*)nullptr, A, C.nbr, C.dx, C.bc, R.nbr, Guides{T},
-                               xp, s + slot(tid), v, [&](int f) {
-                                 return f == 0 ? a.w : f == 1 ? a.e : f == 2 ? a.s : f == 3 ? a.n
-                                        : f == 4 ? a.b : a.t;
-                               });
-      };
       if (R.u[7] != 0.0)
-        cells<NV, JAC>(T, X, Row(R.u, JAC), w, yb, omega, acc, cf);
+        cells<NV, JAC>(T, X, Row(R.u, JAC), w, yb, omega, acc);
       else
-        cells<NV, JAC>(T, X, Rows{A + (size_t)blk * 7 * BLOCK_CELLS + slot(tid)}, w, yb, omega, acc, cf);
+        cells<NV, JAC>(T, X, Rows{A + (size_t)blk * 7 * BLOCK_CELLS + slot(tid)}, w, yb, omega, acc);
       // the next block's loads are in flight over the sums (and pushes)
       if (!JAC && next >= 0) L.load(X, x, next, S.rec[(n + 1) % 3].nbr, C.gin);
       // the warp sums alternate between two buffers: block n + 2 writes its
@@ -269,12 +257,8 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const ET* __restrict__ x,
             tot[v] = cross_block_sum(C.partials + (size_t)v * C.capacity + first, cnt, S.ws[k][0]);
           if (tid == 0) {
             SolveState* St = C.inst.st + li;
-            if (C.fin) {  // the FP64 solver
-              finalize(St, tot[0], C.fin, 0);
-              if (NV == 2) finalize(St, tot[1], FIN_BI_TT, 0);
-            } else if (!JAC) {
-              mx_finalize(St, tot, NV == 1 ? FIN_MX_ALPHA : FIN_MX_GAMMA);
-            }
+            finalize(St, tot[0], C.fin, 0);
+            if (NV == 2) finalize(St, tot[1], FIN_BI_TT, 0);
             St->ticket = 0;
             __threadfence();
           }
@@ -288,12 +272,9 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const ET* __restrict__ x,
     // Copies that may still be on their way into this CTA's shared memory:
     // block n's and n + 1's records and block n's w0 (a step issues the ones
     // after them only once its waits have succeeded).
-    bool drained = true;
-    if (fetch) {
-      drained = async::mbar_drain(&S.wbar[n & 1], (n >> 1) & 1);
-      drained = async::mbar_drain(&S.rbar[n % 3], (n / 3) & 1) && drained;
-      if (ahead) drained = async::mbar_drain(&S.rbar[(n + 1) % 3], ((n + 1) / 3) & 1) && drained;
-    }
+    bool drained = async::mbar_drain(&S.wbar[n & 1], (n >> 1) & 1);
+    drained = async::mbar_drain(&S.rbar[n % 3], (n / 3) & 1) && drained;
+    if (ahead) drained = async::mbar_drain(&S.rbar[(n + 1) % 3], ((n + 1) / 3) & 1) && drained;
     // stop every instance of this CTA's chunk and of its later candidates
     const int where = ROLE_MATVEC | (drained ? 0 : async::ROLE_DRAIN);
     auto stop = [&](int i) {
@@ -309,26 +290,12 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const ET* __restrict__ x,
   }
 }
 
-template <int NV, bool CF, typename ET, bool JAC, int SRC>
-void launch(cudaStream_t s, const MixCtx& C, int count, const ET* x, const double* A, double* y,
-            const double* w0, double omega) {
-  auto kernel = matvec_block_kernel<NV, CF, ET, JAC, SRC>;
+template <int NV, bool JAC>
+void launch(cudaStream_t s, const MixCtx& C, int count, const double* x, const double* A,
+            double* y, const double* w0, double omega) {
+  auto kernel = C.gin ? matvec_block_kernel<NV, JAC, PUSHED> : matvec_block_kernel<NV, JAC, PULL>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
   kernel<<<count, NT, sizeof(Smem), s>>>(C, x, A, y, w0, omega);
-}
-
-template <typename ET>
-void matvec(cudaStream_t s, const MixCtx& C, int count, int ndot, const ET* x, const double* A,
-            double* y, const double* w0) {
-  if (C.cf)
-    ndot == 1 ? launch<1, true, ET, false, PULL>(s, C, count, x, A, y, w0, 0.0)
-              : launch<2, true, ET, false, PULL>(s, C, count, x, A, y, w0, 0.0);
-  else if (C.gin)
-    ndot == 1 ? launch<1, false, ET, false, PUSHED>(s, C, count, x, A, y, w0, 0.0)
-              : launch<2, false, ET, false, PUSHED>(s, C, count, x, A, y, w0, 0.0);
-  else
-    ndot == 1 ? launch<1, false, ET, false, PULL>(s, C, count, x, A, y, w0, 0.0)
-              : launch<2, false, ET, false, PULL>(s, C, count, x, A, y, w0, 0.0);
 }
 
 }  // namespace
@@ -340,22 +307,16 @@ int matvec_block_grid() {
   return 2 * std::max(1, sms);
 }
 
-void launch_matvec_block(cudaStream_t s, const MixCtx& C, int count, int ndot, const void* x,
-                         const double* A, double* y, const double* w0, bool d64) {
-  if (d64)
-    matvec(s, C, count, ndot, static_cast<const double*>(x), A, y, w0);
-  else
-    matvec(s, C, count, ndot, static_cast<const float*>(x), A, y, w0);
+void launch_matvec_block(cudaStream_t s, const MixCtx& C, int count, int ndot, const double* x,
+                         const double* A, double* y, const double* w0) {
+  ndot == 1 ? launch<1, false>(s, C, count, x, A, y, w0, 0.0)
+            : launch<2, false>(s, C, count, x, A, y, w0, 0.0);
 }
 
 void launch_jacobi_block(cudaStream_t s, const MixCtx& C, int count, bool dot, const double* x,
                          const double* A, const double* b, double* y, double omega) {
-  if (C.gin)
-    dot ? launch<1, false, double, true, PUSHED>(s, C, count, x, A, y, b, omega)
-        : launch<0, false, double, true, PUSHED>(s, C, count, x, A, y, b, omega);
-  else
-    dot ? launch<1, false, double, true, PULL>(s, C, count, x, A, y, b, omega)
-        : launch<0, false, double, true, PULL>(s, C, count, x, A, y, b, omega);
+  dot ? launch<1, true>(s, C, count, x, A, y, b, omega)
+      : launch<0, true>(s, C, count, x, A, y, b, omega);
 }
 
 }  // namespace ffvgpu

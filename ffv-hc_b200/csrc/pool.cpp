@@ -262,12 +262,10 @@ MixCtx krylov_mix_ctx(const ffvgpu_pool* P, int fin) {
   return C;
 }
 
-// CTAs of the pipelined kernel.
+// CTAs of the A*x and Jacobi kernels.
 int krylov_grid(ffvgpu_pool* P) {
-  if (!P->grid_mvpipe) {
-    P->grid_mvpipe = matvec_block_grid();
-  }
-  return P->grid_cap > 0 && P->grid_cap < P->grid_mvpipe ? P->grid_cap : P->grid_mvpipe;
+  if (!P->grid_krylov) P->grid_krylov = matvec_block_grid();
+  return P->grid_cap > 0 && P->grid_cap < P->grid_krylov ? P->grid_cap : P->grid_krylov;
 }
 
 // q = A x and q.w (fin FIN_BI_QR0 or FIN_CG_QP), or with t.t as well
@@ -276,7 +274,7 @@ void krylov_matvec(ffvgpu_pool* P, const double* x, double* q, const double* w, 
                    bool two, const double* gin) {
   MixCtx C = krylov_mix_ctx(P, fin);
   C.gin = gin;
-  launch_mx_matvec(P->stream, C, krylov_grid(P), two ? 2 : 1, 0, 0, x, P->A, q, w, true);
+  launch_matvec_block(P->stream, C, krylov_grid(P), two ? 2 : 1, x, P->A, q, w);
 }
 
 // The Jacobi passes after the one from zero: z[0] holds that one's result and

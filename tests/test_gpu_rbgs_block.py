@@ -42,7 +42,7 @@ def test_quotients_at_the_ends_of_the_range(scale):
     compare(*problem(2), 3, scale)
 
 
-@pytest.mark.parametrize("solver", ["rbgs", "cg", "bicgstab"])
+@pytest.mark.parametrize("solver", ["rbgs", "cg", "bicgstab", "mixed", "mixed 1 pass", "mixed 4 passes"])
 def test_one_sided_neighbour_table(solver):
     """Guides are pushed to neighbours only where every face record is matched by the
     neighbour's; with a block that names a neighbour which does not name it (it has the
@@ -70,7 +70,8 @@ def test_one_sided_neighbour_table(solver):
         p.fill("X", 0.0)
         r.append(p.solve_rbgs(1.0, 8, 0.0) if solver == "rbgs" else
                  p.solve_cg(1.0, 3, 8, 0.0) if solver == "cg" else
-                 p.solve_bicgstab(1.0, 2, 8, 0.0))
+                 p.solve_bicgstab(1.0, 2, 8, 0.0) if solver == "bicgstab" else
+                 p.solve_mixed(1.5, 8, {"mixed": 4, "mixed 1 pass": 8}.get(solver, 2), 6, 0.0))
     assert_bitwise(r[1]["history"], r[0]["history"], "history")
     assert_bitwise(interior(Q.download("X", VC))[:g.nb], interior(P.download("X", VC)), "x")
     P.close()
