@@ -197,7 +197,7 @@ jacobi_kernel(KCtx C, double* __restrict__ xout, const double* __restrict__ A,
 
 // r = b - A x (calc_r, bils.f90:208-254); x guides from 'gst' when given.
 __global__ void __launch_bounds__(THREADS, 3)
-calc_r_kernel(KCtx C, const double* __restrict__ x, const double* __restrict__ gst,
+calc_r_kernel(const __grid_constant__ KCtx C, const double* __restrict__ x, const double* __restrict__ gst,
               const double* __restrict__ A, const double* __restrict__ bvec,
               double* __restrict__ rout, SolveState* st) {
   if (st && solve_done(st)) return;
@@ -304,15 +304,24 @@ shift_kernel(double* __restrict__ x, SolveState* st) {
 // Exchange into a stored guide layer, layout conversion and set-up kernels.
 // ---------------------------------------------------------------------------
 
-// Writes layer-1 guide values of every face of every block into g.
+// Writes layer-1 guide values of every face of every block into g, as pairs of
+// positions of a face (guide_pair: the loads of both in flight, coordinates by
+// selects) with three pairs per thread.  1164 blocks: 30.4 us one value at a
+// time through guide_value, whose axis-indexed coordinates live in local memory,
+// 15.0 us here.
 __global__ void __launch_bounds__(THREADS)
-exchange_kernel(KCtx C, const double* __restrict__ x, double* __restrict__ g) {
-  const int blk = C.first + blockIdx.x, tid = threadIdx.x;
-  const int a = tid & 15, b = tid >> 4;
-  for (int f = 0; f < 6; ++f) {
+exchange_kernel(const __grid_constant__ KCtx C, const double* __restrict__ x,
+                double* __restrict__ g) {
+  const int blk = C.first + blockIdx.x, tid = threadIdx.x, p0 = tid & 127, p1 = p0 + 128;
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    const int f = 2 * r + (tid >> 7);
     const FaceNbr nb = C.nbr[blk * 6 + f];
-    g[((size_t)blk * 6 + f) * FACE_CELLS + b * 16 + a] =
-        guide_value(x, blk, f, a, b, 1, nb, C.bc, C.dx[blk]);
+    double v0, v1;
+    guide_pair(x, blk, f, p0, p1, nb, C.bc, C.dx[blk], v0, v1);
+    double* gf = g + ((size_t)blk * 6 + f) * FACE_CELLS;
+    gf[p0] = v0;
+    gf[p1] = v1;
   }
 }
 
@@ -424,7 +433,7 @@ unpack_flag_kernel(const uint8_t* __restrict__ flags, int vc, int32_t* __restric
 // Colour-split interior -> host layout, with vc guide layers per face
 // computed as the reference's exchange + outer BC would (layers 1..vc).
 __global__ void __launch_bounds__(THREADS)
-unpack_kernel(KCtx C, const double* __restrict__ src, size_t stride, int vc, int with_guides,
+unpack_kernel(const __grid_constant__ KCtx C, const double* __restrict__ src, size_t stride, int vc, int with_guides,
               double* __restrict__ stage) {
   const int blk = C.first + blockIdx.x, tid = threadIdx.x;
   const int w = 16 + 2 * vc;
@@ -532,7 +541,7 @@ assemble_kernel(KCtx C, const double* __restrict__ ux, const double* __restrict_
 // with its stored guide layer.  Each expression in the reference's order.
 template <bool CORR>
 __global__ void __launch_bounds__(THREADS)
-projection_kernel(KCtx C, const double* __restrict__ p, const double* __restrict__ gp,
+projection_kernel(const __grid_constant__ KCtx C, const double* __restrict__ p, const double* __restrict__ gp,
                   const double* __restrict__ cut, const uint8_t* __restrict__ flags,
                   double* __restrict__ ux, double* __restrict__ uy, double* __restrict__ uz,
                   double* __restrict__ vface, double* __restrict__ lapp, double rhof, double dt,
@@ -542,6 +551,11 @@ projection_kernel(KCtx C, const double* __restrict__ p, const double* __restrict
   stage_tile(xs, p, blk, C, gp);
   __syncthreads();
   const double dx = C.dx[blk];
+  // two cells' loads in flight where there are 28 arrays to read and write (1164
+  // blocks: 395 -> 313 us; remove_p's 11 are faster one cell at a time, 115 us
+  // against 151)
+  constexpr int UNROLL = CORR ? 2 : 1;
+#pragma unroll UNROLL
   for (int m = 0; m < 16; ++m) {
     const int s = tid + THREADS * m;
     int i, j, k;
@@ -640,11 +654,17 @@ urec_kernel(const double* __restrict__ A, double* __restrict__ urec,
             int32_t* __restrict__ ucount) {
   const int blk = blockIdx.x, tid = threadIdx.x;
   const double* Ab = A + (size_t)blk * 7 * BLOCK_CELLS;
-  bool same = true;
-  for (int m = 0; m < 16; ++m)
-    for (int a = 0; a < 7; ++a)
-      same = same && __double_as_longlong(Ab[(size_t)a * BLOCK_CELLS + tid + THREADS * m]) ==
-                         __double_as_longlong(Ab[(size_t)a * BLOCK_CELLS]);
+  // every value is compared, many loads in flight (1164 blocks: 42 us; 59 us
+  // with a test that stops at the first difference, waiting for each load)
+  long long diff = 0;
+#pragma unroll
+  for (int a = 0; a < 7; ++a) {
+    const long long c0 = __double_as_longlong(__ldg(Ab + (size_t)a * BLOCK_CELLS));
+#pragma unroll
+    for (int m = 0; m < 16; ++m)
+      diff |= __double_as_longlong(__ldg(Ab + (size_t)a * BLOCK_CELLS + tid + THREADS * m)) ^ c0;
+  }
+  bool same = diff == 0;
   same = __syncthreads_and(same);
   if (tid < 8) urec[(size_t)blk * 8 + tid] = tid < 7 ? Ab[(size_t)tid * BLOCK_CELLS] : (same ? 1.0 : 0.0);
   if (tid == 0 && same) atomicAdd(ucount, 1);

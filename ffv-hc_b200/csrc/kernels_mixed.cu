@@ -238,27 +238,32 @@ mx_pack_kernel(int first, const double* __restrict__ A, uint32_t* __restrict__ c
   const double* Ab = A + (size_t)blk * 7 * BLOCK_CELLS;
   uint32_t* cb = D64 ? nullptr : coef + (size_t)blk * COEF_WORDS;
   double* cd = D64 ? coef64 + (size_t)blk * COEF_WORDS : nullptr;
+  // uniform block: all seven coefficients bitwise equal to cell 0's everywhere.
+  // Each value is read once, for the words and for the comparison.
+  double c0[7];
+#pragma unroll
+  for (int a = 0; a < 7; ++a) c0[a] = __ldg(Ab + a * BLOCK_CELLS);
+  long long diff = 0;
+#pragma unroll 4
   for (int w = threadIdx.x; w < BLOCK_CELLS; w += MT) {
     const int m = w / PTS, t = w % PTS;
     const int s = sweep_cell<PTS>(t, m);
+    double v[7];
+#pragma unroll
+    for (int a = 0; a < 7; ++a) v[a] = __ldg(Ab + a * BLOCK_CELLS + s);
+#pragma unroll
+    for (int a = 0; a < 7; ++a) diff |= __double_as_longlong(v[a]) ^ __double_as_longlong(c0[a]);
     if (D64) {
 #pragma unroll
-      for (int a = 0; a < 6; ++a) cd[(a * CPT + m) * PTS + t] = Ab[(1 + a) * BLOCK_CELLS + s];
-      cd[(6 * CPT + m) * PTS + t] = 1.0 / Ab[s];
+      for (int a = 0; a < 6; ++a) cd[(a * CPT + m) * PTS + t] = v[1 + a];
+      cd[(6 * CPT + m) * PTS + t] = 1.0 / v[0];
     } else {
 #pragma unroll
-      for (int a = 0; a < 6; ++a)
-        cb[coef_word<PTS>(a, m, t)] = hi_round(Ab[(1 + a) * BLOCK_CELLS + s]);
-      cb[coef_word<PTS>(6, m, t)] = hi_round(1.0 / Ab[s]);
+      for (int a = 0; a < 6; ++a) cb[coef_word<PTS>(a, m, t)] = hi_round(v[1 + a]);
+      cb[coef_word<PTS>(6, m, t)] = hi_round(1.0 / v[0]);
     }
   }
-  // uniform block: all seven coefficients bitwise equal to cell 0's everywhere
-  bool same = true;
-  for (int s = threadIdx.x; s < BLOCK_CELLS; s += MT)
-#pragma unroll
-    for (int a = 0; a < 7; ++a)
-      same = same && __double_as_longlong(Ab[a * BLOCK_CELLS + s]) ==
-                         __double_as_longlong(Ab[a * BLOCK_CELLS]);
+  bool same = diff == 0;
   same = __syncthreads_and(same);
   if (threadIdx.x < 8)
     ucoef[(size_t)blk * 8 + threadIdx.x] =
