@@ -1023,17 +1023,17 @@ def main():
     e2e_value = whole_job_rate(world, cells * args.sweeps * args.steps, te_ms)
 
     # ---- roofline of the dominant kernel (fused residual + RB sweep) ---------
-    # achieved: the fixed algorithmic bytes of an RB sweep with its residual,
-    # 80 B per interior cell (7 coefficients + b + x read, x written), over
-    # the kernel's average launch; 'traffic' is what the kernel moves from
-    # DRAM (ncu), below the algorithmic bytes because a uniform block's seven
-    # coefficients come from one record (its pass moves 24 B per cell)
+    # achieved: the bytes a pass must move in the pool's format -- 80 B per
+    # interior cell (7 coefficients + b + x read, x written), 24 B in a block
+    # whose seven coefficients come from one record -- over the kernel's average
+    # launch; alg_gbs counts 80 B in every cell; 'traffic' is what the kernel
+    # moves from DRAM (ncu)
     avg_launch_ms = float(np.sum(sweep_ms) / max(1, np.sum(sweep_n)))
     ublocks = int(r.get("uniform_blocks", 0))
     alg_bytes = BYTES_PER_SWEEP_CELL * cells
     fmt_bytes = CELLS_PER_BLOCK * ((g.nb - ublocks) * BYTES_PER_SWEEP_CELL +
                                    ublocks * BYTES_PER_SWEEP_CELL_UNIFORM)
-    achieved = alg_bytes / (avg_launch_ms * 1e-3) / 1e9
+    achieved = fmt_bytes / (avg_launch_ms * 1e-3) / 1e9
     peak, peak_kind = measured_peaks()
     traffic, traffic_src = profile_traffic(args.level, cells, fmt_bytes)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -1044,7 +1044,7 @@ def main():
                 "format_bytes_per_launch": fmt_bytes,
                 "format_bytes_per_cell": f"{BYTES_PER_SWEEP_CELL} (per-cell coefficients), "
                                          f"{BYTES_PER_SWEEP_CELL_UNIFORM} (uniform block)",
-                "format_gbs": fmt_bytes / (avg_launch_ms * 1e-3) / 1e9,
+                "alg_gbs": alg_bytes / (avg_launch_ms * 1e-3) / 1e9,
                 "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)"}
 
     cpu = None
