@@ -34,12 +34,6 @@ __device__ __forceinline__ int guide_at(int face, int p) {
                    : face < 4 ? (v + 1) * TP + (out + 1) * TR + (u >> 1)
                               : (out + 1) * TP + (v + 1) * TR + (u >> 1));
 }
-// The first guide layer read as [face][p].
-struct Guides {
-  const double* T;
-  __device__ double operator[](int g) const { return T[guide_at(g >> 8, g & 255)]; }
-};
-
 // A CTA of 256 threads holds one block.  Thread t has (j, i / 2) = t & 127 and
 // of the planes k the pairs 4 m + 2 h + e (h = t >> 7; e = 0, 1; m = 0..3), both
 // colours, in registers: X[c][2 m + e] is storage slot slot(t) + c * 2048 +
@@ -127,7 +121,7 @@ struct Staging {
 // of an x face touches 32 lines of the 28 KB that two CTAs' shared memory leaves
 // to L1, so those loads, and the interior's behind them, wait for lines: reading
 // all guides from the neighbours made an RBGS pass of the level-5 sphere grid
-// 176 us, pushing these 151 us (without any guides 125 us).
+// 176 us, pushing these 147 us (without any guides 125 us).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double cell(const double* T, int i, int j, int k) {
   return T[((i + j + k) & 1) * TH + (k + 1) * TP + (j + 1) * TR + (i >> 1)];

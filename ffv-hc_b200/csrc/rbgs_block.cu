@@ -18,7 +18,7 @@
 // time.  Level-5 sphere grid (4692 blocks, 4256 uniform), per pass: 238 us for
 // a persistent kernel with one cell per consumer thread and stencil
 // neighbours chosen by selects (500 MB of coefficients and b through a TMA
-// ring), 151 us here; a copy of x through the same structure takes 86 us, the
+// ring), 147 us here; a copy of x through the same structure takes 86 us, the
 // pass without guide layers 125 us.  72 blocks: 18.0 -> 13.7 us; 324: 33 ->
 // 25.7 us.  Tried and slower at level 5 (us per pass): 128 threads with whole
 // k columns in registers 199; 512 threads on strided planes, one CTA per SM
@@ -28,7 +28,6 @@
 #include <cfloat>
 #include <cstddef>
 #include <cstdint>
-#include <cstdlib>
 #include <mutex>
 #include <type_traits>
 #include <cuda_runtime.h>
