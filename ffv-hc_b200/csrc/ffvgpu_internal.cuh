@@ -116,21 +116,45 @@ static __device__ __noinline__ double guide_value(const T* __restrict__ x, int b
   }
 }
 
+// How a kernel reads a field.  ReadOnly: through the read-only path, for memory
+// that nothing writes while the kernel is resident.  Written: for a kernel
+// launched as a programmatic dependent of the one that writes the field, which
+// is resident while that one still writes; the read-only path is not defined
+// there, and the compiler may move such loads above the wait for the writer.
+// These are ordinary loads that stay below it.
+struct ReadOnly {
+  template <typename T>
+  __device__ __forceinline__ static T ld(const T* p) {
+    return __ldg(p);
+  }
+};
+struct Written {
+  __device__ __forceinline__ static double ld(const double* p) {
+#ifdef __CUDA_ARCH__
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+#else
+    return *p;
+#endif
+  }
+};
+
 // The eight cells (i..i+1, j..j+1, k..k+1) of block blk: nnn, pnn, npn, nnp,
 // npp, pnp, ppn, ppp (first letter: +1 along i, then j, then k).
-template <typename T>
-__device__ __forceinline__ void load8(const T* __restrict__ x, int blk, int i, int j, int k,
+template <typename LD, typename T>
+__device__ __forceinline__ void load8(const T* x, int blk, int i, int j, int k,
                                       double (&a)[8]) {
   const T* b = x + (size_t)blk * BLOCK_CELLS + (k * 16 + j) * 8;
   const int e = ((i + j + k) & 1) << 11, o = e ^ HALF_CELLS, h0 = i >> 1, h1 = (i + 1) >> 1;
-  a[0] = (double)__ldg(b + e + h0);
-  a[1] = (double)__ldg(b + o + h1);
-  a[2] = (double)__ldg(b + o + 8 + h0);
-  a[3] = (double)__ldg(b + o + 128 + h0);
-  a[4] = (double)__ldg(b + e + 136 + h0);
-  a[5] = (double)__ldg(b + e + 128 + h1);
-  a[6] = (double)__ldg(b + e + 8 + h1);
-  a[7] = (double)__ldg(b + o + 136 + h1);
+  a[0] = (double)LD::ld(b + e + h0);
+  a[1] = (double)LD::ld(b + o + h1);
+  a[2] = (double)LD::ld(b + o + 8 + h0);
+  a[3] = (double)LD::ld(b + o + 128 + h0);
+  a[4] = (double)LD::ld(b + e + 136 + h0);
+  a[5] = (double)LD::ld(b + e + 128 + h1);
+  a[6] = (double)LD::ld(b + e + 8 + h1);
+  a[7] = (double)LD::ld(b + o + 136 + h1);
 }
 
 // Guide cell (layer 1) at position p (u + 16 v) of a 2:1 face, in two steps
@@ -156,11 +180,10 @@ struct CoarseGuide {  // interpolation from a coarse neighbour (sup.f90:54-120)
     j = (axis == 0 ? iu : axis == 1 ? ia : iv) - 1;
     k = (axis == 2 ? ia : iv) - 1;
   }
-  template <typename T>
-  __device__ __forceinline__ void load(const T* __restrict__ x, int face, int p,
-                                       const FaceNbr& nb) {
+  template <typename LD, typename T>
+  __device__ __forceinline__ void load(const T* x, int face, int p, const FaceNbr& nb) {
     at(face, p, nb);
-    load8(x, blk, i, j, k, a);
+    load8<LD>(x, blk, i, j, k, a);
   }
   __device__ __forceinline__ double value() const {
     return (1.0 - t) * ((1.0 - s) * ((1.0 - r) * a[0] + r * a[1]) +
@@ -181,11 +204,10 @@ struct FineGuide {  // mean of eight cells of a fine neighbour (sup.f90:122-179)
     j = axis == 0 ? lu : axis == 1 ? la : lv;
     k = axis == 2 ? la : lv;
   }
-  template <typename T>
-  __device__ __forceinline__ void load(const T* __restrict__ x, int face, int p,
-                                       const FaceNbr& nb) {
+  template <typename LD, typename T>
+  __device__ __forceinline__ void load(const T* x, int face, int p, const FaceNbr& nb) {
     at(face, p, nb);
-    load8(x, blk, i, j, k, a);
+    load8<LD>(x, blk, i, j, k, a);
   }
   __device__ __forceinline__ double value() const {
     return 0.125 * (a[0] + a[1] + a[2] + a[3] + a[4] + a[5] + a[6] + a[7]);
@@ -211,27 +233,27 @@ __device__ __forceinline__ double outer_guide(double x0, int face, const BCSet& 
 // [0, 256) (p = v*16 + u), with every load of both issued before any is
 // used: the batched form of guide_value for the pipelined kernels.  Same
 // expressions, same evaluation order, same results as guide_value.
-template <typename T>
-__device__ __forceinline__ void guide_pair(const T* __restrict__ x, int blk, int face,
-                                           int p0, int p1, const FaceNbr& nb, const BCSet& bc,
-                                           double dx, double& v0, double& v1) {
+template <typename LD = ReadOnly, typename T>
+__device__ __forceinline__ void guide_pair(const T* x, int blk, int face, int p0, int p1,
+                                           const FaceNbr& nb, const BCSet& bc, double dx,
+                                           double& v0, double& v1) {
   if (nb.kind == NB_COARSE) {
     CoarseGuide g0, g1;
-    g0.load(x, face, p0, nb);
-    g1.load(x, face, p1, nb);
+    g0.load<LD>(x, face, p0, nb);
+    g1.load<LD>(x, face, p1, nb);
     v0 = g0.value();
     v1 = g1.value();
   } else if (nb.kind == NB_FINE) {
     FineGuide g0, g1;
-    g0.load(x, face, p0, nb);
-    g1.load(x, face, p1, nb);
+    g0.load<LD>(x, face, p0, nb);
+    g1.load<LD>(x, face, p1, nb);
     v0 = g0.value();
     v1 = g1.value();
   } else {
     const bool own = nb.kind == NB_OUTER;
     const T* s = x + (size_t)(own ? blk : nb.id[0]) * BLOCK_CELLS;
-    v0 = (double)__ldg(s + face_slot(face, p0, own));
-    v1 = (double)__ldg(s + face_slot(face, p1, own));
+    v0 = (double)LD::ld(s + face_slot(face, p0, own));
+    v1 = (double)LD::ld(s + face_slot(face, p1, own));
     if (own) {
       v0 = outer_guide(v0, face, bc, dx);
       v1 = outer_guide(v1, face, bc, dx);

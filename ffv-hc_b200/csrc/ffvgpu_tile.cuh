@@ -56,38 +56,37 @@ __host__ __device__ constexpr bool is_pushed(int f, int kind) {
 }
 
 // Loads of a block's interior and guide layer into registers, all in flight
-// together but (PULL) those of 2:1 faces.
-template <int SRC>
+// together but (PULL) those of 2:1 faces.  LD: how x and gst are read (Written in
+// kernels launched as programmatic dependents of the one that wrote them).
+template <int SRC, typename LD>
 struct Staging {
   double g[3][2];
-  template <typename ET>
-  __device__ __forceinline__ void load(double (&X)[2][NC], const ET* __restrict__ x, int blk,
-                                       const FaceNbr* nb, const double* __restrict__ gst) {
+  __device__ __forceinline__ void load(double (&X)[2][NC], const double* x, int blk,
+                                       const FaceNbr* nb, const double* gst) {
     const int t = threadIdx.x, p = t & 127;
-    const ET* xb = x + (size_t)blk * BLOCK_CELLS + slot(t);
+    const double* xb = x + (size_t)blk * BLOCK_CELLS + slot(t);
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int n = 0; n < NC; ++n) X[c][n] = (double)__ldg(xb + c * HALF_CELLS + plane(n) * 128);
+      for (int n = 0; n < NC; ++n) X[c][n] = LD::ld(xb + c * HALF_CELLS + plane(n) * 128);
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
       const int f = 2 * r + (t >> 7), kind = nb[f].kind;
       if (SRC == STORED || (SRC == PUSHED && is_pushed(f, kind))) {
         const double* gs = gst + ((size_t)blk * 6 + f) * FACE_CELLS + p;
-        g[r][0] = __ldg(gs);
-        g[r][1] = __ldg(gs + 128);
+        g[r][0] = LD::ld(gs);
+        g[r][1] = LD::ld(gs + 128);
       } else if (kind <= NB_SAME) {
         const bool outer = kind == NB_OUTER;
-        const ET* s = x + (size_t)(outer ? blk : nb[f].id[0]) * BLOCK_CELLS;
-        g[r][0] = (double)__ldg(s + face_slot(f, p, outer));
-        g[r][1] = (double)__ldg(s + face_slot(f, p + 128, outer));
+        const double* s = x + (size_t)(outer ? blk : nb[f].id[0]) * BLOCK_CELLS;
+        g[r][0] = LD::ld(s + face_slot(f, p, outer));
+        g[r][1] = LD::ld(s + face_slot(f, p + 128, outer));
       }
     }
   }
-  template <typename ET>
-  __device__ __forceinline__ void put(double* T, const double (&X)[2][NC],
-                                      const ET* __restrict__ x, int blk, const FaceNbr* nb,
-                                      const BCSet& bc, const double* __restrict__ dxs) {
+  __device__ __forceinline__ void put(double* T, const double (&X)[2][NC], const double* x,
+                                      int blk, const FaceNbr* nb, const BCSet& bc,
+                                      const double* __restrict__ dxs) {
     const int t = threadIdx.x, p = t & 127;
 #pragma unroll
     for (int c = 0; c < 2; ++c)
@@ -103,7 +102,7 @@ struct Staging {
           g[r][0] = outer_guide(g[r][0], f, bc, dx);
           g[r][1] = outer_guide(g[r][1], f, bc, dx);
         } else if (SRC == PULL && kind != NB_SAME) {
-          guide_pair(x, blk, f, p, p + 128, nb[f], bc, 0.0, g[r][0], g[r][1]);
+          guide_pair<LD>(x, blk, f, p, p + 128, nb[f], bc, 0.0, g[r][0], g[r][1]);
         }
       }
       T[guide_at(f, p)] = g[r][0];

@@ -165,7 +165,7 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const double* __restrict__
     return async::mbar_wait(&S.rbar[m % 3], (m / 3) & 1, &S.abort_flag, ROLE_MATVEC, C.wait_ns);
   };
   double X[2][NC];
-  Staging<SRC> L;
+  Staging<SRC, ReadOnly> L;
   int n = 0;      // blocks of this CTA so far
   int run = 0;    // thread 0: blocks of the current instance not yet on its ticket
   int ahead = 0;  // whether block n + 1's record has been fetched

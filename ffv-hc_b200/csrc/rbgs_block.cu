@@ -188,9 +188,9 @@ static_assert(2 * (sizeof(Smem) + 1024) <= 228 * 1024, "two CTAs per SM");
 
 template <bool RES, bool SWEEP, int SRC, int PER_SM>
 __global__ void __launch_bounds__(NT, PER_SM)
-rbgs_block_kernel(const __grid_constant__ KCtx C, const double* __restrict__ xin,
+rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
                   double* __restrict__ xout, const double* __restrict__ A,
-                  const double* __restrict__ bvec, const double* __restrict__ gst,
+                  const double* __restrict__ bvec, const double* gst,
                   double* __restrict__ gout, double omega, double* __restrict__ partials,
                   SolveState* st, int fin, int iter,
                   const int32_t* __restrict__ order) {
@@ -241,7 +241,7 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* __restrict__ xin
   int n = 0;
   if (skip) blk = -1;  // the copies in flight are drained below
   double X[2][NC];
-  Staging<SRC> L;
+  Staging<SRC, Written> L;  // the pass before may still be writing while this one starts
   if (ok && blk >= 0) L.load(X, xin, blk, S.rec[0].nbr, gst);
   while (blk >= 0) {
     const int k = n & 1;
