@@ -85,6 +85,11 @@ void launch_mx_matvec(cudaStream_t s, const MixCtx& C, int count, int ndot, int 
 void launch_matvec_block(cudaStream_t s, const MixCtx& C, int count, int ndot, const double* x,
                          const double* A, double* y, const double* w0);
 int matvec_block_grid();
+// A Jacobi pass as launch_jacobi_block's on the pipelined kernel (its tile and
+// coefficient ring, b in the dot partner's place): 'count' CTAs of mx_grid_sizes'
+// mvpipe.  launch_mx_matvec with C.fin is the FP64 solvers' A x on it.
+void launch_jacobi_pipe(cudaStream_t s, const MixCtx& C, int count, bool dot, const double* x,
+                        const double* A, const double* b, double* y, double omega);
 void launch_jacobi_block(cudaStream_t s, const MixCtx& C, int count, bool dot, const double* x,
                          const double* A, const double* b, double* y, double omega);
 // Coarse-fine flux mismatch per face cell of the (block, face) pairs

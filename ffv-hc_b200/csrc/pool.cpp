@@ -198,6 +198,15 @@ ffvgpu_status ensure_urec(ffvgpu_pool* P) {
   return FFVGPU_OK;
 }
 
+// The count of uniform blocks, read back once per assembled A.
+ffvgpu_status read_ucount(ffvgpu_pool* P) {
+  if (P->ucount_version != P->sys_version) {
+    CK(download_sync(P, &P->ucount_h, P->ucount_d, sizeof(int32_t)));
+    P->ucount_version = P->sys_version;
+  }
+  return FFVGPU_OK;
+}
+
 // The guide buffers that RBGS passes push into, for a neighbour table in which
 // every face is the other side's neighbour too (a shard's halo faces are not).
 ffvgpu_status ensure_push(ffvgpu_pool* P) {
@@ -262,34 +271,79 @@ MixCtx krylov_mix_ctx(const ffvgpu_pool* P, int fin) {
   return C;
 }
 
-// CTAs of the A*x and Jacobi kernels.
-int krylov_grid(ffvgpu_pool* P) {
+// What a Krylov solve's A*x and Jacobi passes run on.  ring: the pipelined
+// kernel of the mixed form (one CTA per SM, coefficients through a ring of bulk
+// copies, guides from the neighbours' interiors); else matvec_block.cu (two
+// smaller CTAs per SM, which read coefficients as they use them, guides pushed
+// into g by the kernel that makes the operand).
+struct KrylovForm {
+  bool ring = false;
+  int grid = 0;
+  double* g[2] = {nullptr, nullptr};
+};
+
+// The ring keeps a varied block's 224 KB of coefficients streaming at HBM speed
+// (all 4692 blocks varied: A x 250 us a launch, a Jacobi pass 245; 238 at the
+// measured peak), but its one CTA per SM is the slower one where most blocks
+// are uniform.  us per CG iteration, PreCount 2, blocks /
+// ring, by the share of varied blocks:
+//    324 blocks: 0.3: 83 / 86,   0.8: 100 / 100,  1: 121 / 107
+//    548 blocks: 0.3: 128 / 127, 0.5: 140 / 134,  1: 188 / 162
+//   1164 blocks: 0.3: 225 / 222, 0.4: 244 / 231,  1: 364 / 281
+//   4692 blocks: 0.3: 741 / 720, 0.4: 824 / 770,  1: 1317 / 1003
+// so the line lies at a third of the pool and more varied blocks than
+// matvec_block.cu has CTAs (BiCGSTAB and the other PreCounts agree).
+ffvgpu_status krylov_form(ffvgpu_pool* P, KrylovForm* F) {
+  ffvgpu_status s;
+  if ((s = ensure_kpipe(P))) return s;
   if (!P->grid_krylov) P->grid_krylov = matvec_block_grid();
-  return P->grid_cap > 0 && P->grid_cap < P->grid_krylov ? P->grid_cap : P->grid_krylov;
+  if (P->nb > P->grid_krylov) {
+    if ((s = read_ucount(P))) return s;
+    const int64_t varied = P->nb - P->ucount_h;
+    F->ring = varied > P->grid_krylov && 100 * varied > 35 * (int64_t)P->nb;
+  }
+  if (F->ring) {
+    if (!P->grid_ring) {
+      int a, b, c, d;
+      mx_grid_sizes(P->m_threads, &a, &b, &c, &d, &P->grid_ring);
+    }
+    F->grid = P->grid_ring;
+  } else {
+    F->grid = P->grid_krylov;
+    if ((s = ensure_push(P))) return s;
+    F->g[0] = P->gpush[0];
+    F->g[1] = P->gpush[1];
+  }
+  if (P->grid_cap > 0 && P->grid_cap < F->grid) F->grid = P->grid_cap;
+  return FFVGPU_OK;
 }
 
 // q = A x and q.w (fin FIN_BI_QR0 or FIN_CG_QP), or with t.t as well
 // (FIN_BI_TS, then FIN_BI_TT) when 'two'.  gin: x's pushed guides (or null).
-void krylov_matvec(ffvgpu_pool* P, const double* x, double* q, const double* w, int fin,
-                   bool two, const double* gin) {
+void krylov_matvec(ffvgpu_pool* P, const KrylovForm& F, const double* x, double* q,
+                   const double* w, int fin, bool two, const double* gin) {
   MixCtx C = krylov_mix_ctx(P, fin);
   C.gin = gin;
-  launch_matvec_block(P->stream, C, krylov_grid(P), two ? 2 : 1, x, P->A, q, w);
+  if (F.ring)
+    launch_mx_matvec(P->stream, C, F.grid, two ? 2 : 1, 0, 0, x, P->A, q, w, true);
+  else
+    launch_matvec_block(P->stream, C, F.grid, two ? 2 : 1, x, P->A, q, w);
 }
 
 // The Jacobi passes after the one from zero: z[0] holds that one's result and
-// gpush[0] its guides; returns the buffer with the last one's, whose guides are
-// in gpush[(K - 1) & 1].  With dot the last also forms b.z (FIN_CG_RR1).
-double* krylov_jacobi(ffvgpu_pool* P, double* const z[2], const double* b, int K, double omega,
-                      bool dot, int64_t& words, int64_t& coef, int& launches) {
+// F.g[0] its guides; returns the buffer with the last one's, whose guides are
+// in F.g[(K - 1) & 1].  With dot the last also forms b.z (FIN_CG_RR1).
+double* krylov_jacobi(ffvgpu_pool* P, const KrylovForm& F, double* const z[2], const double* b,
+                      int K, double omega, bool dot, int64_t& words, int64_t& coef,
+                      int& launches) {
   for (int k = 2; k <= K; ++k) {
     const bool last = k == K;
     MixCtx C = krylov_mix_ctx(P, dot && last ? FIN_CG_RR1 : 0);
-    C.gin = P->gpush[k & 1];
+    C.gin = F.g[k & 1];
     // the vector after CG's last pass is not a stencil's operand (p is)
-    C.gout = dot && last ? nullptr : P->gpush[(k - 1) & 1];
-      launch_jacobi_block(P->stream, C, krylov_grid(P), dot && last, z[k & 1], P->A, b,
-                        z[(k - 1) & 1], omega);
+    C.gout = dot && last ? nullptr : F.g[(k - 1) & 1];
+    const auto jacobi = F.ring ? launch_jacobi_pipe : launch_jacobi_block;
+    jacobi(P->stream, C, F.grid, dot && last, z[k & 1], P->A, b, z[(k - 1) & 1], omega);
     words += 10;
     coef += 7;
     launches++;
@@ -411,14 +465,6 @@ ffvgpu_status solve_status(const SolveState& h, const ffvgpu_iter_params* prm, i
 
 int64_t interior_bytes(const ffvgpu_pool* P, int words) {
   return (int64_t)P->nb * (int64_t)BC * 8 * words;
-}
-// The count of uniform blocks, read back once per assembled A.
-ffvgpu_status read_ucount(ffvgpu_pool* P) {
-  if (P->ucount_version != P->sys_version) {
-    CK(download_sync(P, &P->ucount_h, P->ucount_d, sizeof(int32_t)));
-    P->ucount_version = P->sys_version;
-  }
-  return FFVGPU_OK;
 }
 // Bytes of one pass of the red-black kernel: 'words' per cell (10 for a
 // sweep with its residual, 9 for a residual alone) in a block that streams
@@ -1082,7 +1128,8 @@ ffvgpu_status ffvgpu_solve_cg(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   std::memset(&R, 0, sizeof(R));
   if ((s = ensure_hist(P, N > 0 ? N : 1))) return s;
   if ((s = reset_state(P, prm->epsilon, N, P->hist_d))) return s;
-  if ((s = ensure_kpipe(P)) || (s = ensure_push(P))) return s;
+  KrylovForm F;
+  if ((s = krylov_form(P, &F))) return s;
   const KCtx C = P->ctx(P->bc_p);
   const int every = prm->check_every > 0 ? prm->check_every : 16;
   const bool poll = prm->epsilon > 0.0;
@@ -1117,7 +1164,7 @@ ffvgpu_status ffvgpu_solve_cg(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   CK(cudaEventRecord(P->ev2, P->stream));
   const int launches_before = launches;
   if (K > 1) {
-    launch_jacobi_zero(P->stream, C, P->r, P->A, P->z[0], prm->omega, P->gpush[0], P->st);
+    launch_jacobi_zero(P->stream, C, P->r, P->A, P->z[0], prm->omega, F.g[0], P->st);
     launches++;
     words += 9;
     coef += 7;
@@ -1131,14 +1178,14 @@ ffvgpu_status ffvgpu_solve_cg(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
       coef += 7;
       launches++;
     }
-    double* z = krylov_jacobi(P, P->z, P->r, K, prm->omega, true, words, coef, launches);
-    launch_cg_p(P->stream, C, z, P->p, P->gpush[0], P->st, c);
+    double* z = krylov_jacobi(P, F, P->z, P->r, K, prm->omega, true, words, coef, launches);
+    launch_cg_p(P->stream, C, z, P->p, F.g[0], P->st, c);
     words += c == 1 ? 2 : 3;
-    krylov_matvec(P, P->p, P->q, P->p, FIN_CG_QP, false, P->gpush[0]);  // x, A, w, y
+    krylov_matvec(P, F, P->p, P->q, P->p, FIN_CG_QP, false, F.g[0]);  // x, A, w, y
     words += 10;
     coef += 7;
     launch_cg_update(P->stream, C, x, P->p, P->r, P->q, P->A, K > 1 ? P->z[0] : nullptr,
-                     prm->omega, P->gpush[0], P->kpart, P->st, c);
+                     prm->omega, F.g[0], P->kpart, P->st, c);
     words += 6 + (K > 1 ? 8 : 0);
     coef += K > 1 ? 7 : 0;
     launches += 3;
@@ -1200,7 +1247,8 @@ ffvgpu_status ffvgpu_solve_bicgstab(ffvgpu_pool* P, const ffvgpu_iter_params* pr
   if (!(prm->restart_drop >= 0.0 && prm->restart_drop < 1.0))
     return bad("restart_drop must lie in [0, 1)");
   if ((s = reset_state(P, prm->epsilon, N, P->hist_d, prm->restart_drop))) return s;
-  if ((s = ensure_kpipe(P)) || (s = ensure_push(P))) return s;
+  KrylovForm F;
+  if ((s = krylov_form(P, &F))) return s;
   const KCtx C = P->ctx(P->bc_p);
   const int every = prm->check_every > 0 ? prm->check_every : 16;
   const bool poll = prm->epsilon > 0.0;
@@ -1240,14 +1288,14 @@ ffvgpu_status ffvgpu_solve_bicgstab(ffvgpu_pool* P, const ffvgpu_iter_params* pr
     double* pz = P->z[0];
     double* sz = P->zb[0];
     launch_bicg_p(P->stream, C, P->r, P->p, P->q, P->r0, P->A, K > 0 ? P->z[0] : nullptr,
-                  prm->omega, P->gpush[0], P->st);
-    if (K > 0) pz = krylov_jacobi(P, P->z, P->p, K, prm->omega, false, words, coef, launches);
-    const double* g = K > 0 ? P->gpush[(K - 1) & 1] : nullptr;
-    krylov_matvec(P, pz, P->q, P->r0, FIN_BI_QR0, false, g);
+                  prm->omega, F.g[0], P->st);
+    if (K > 0) pz = krylov_jacobi(P, F, P->z, P->p, K, prm->omega, false, words, coef, launches);
+    const double* g = K > 0 ? F.g[(K - 1) & 1] : nullptr;
+    krylov_matvec(P, F, pz, P->q, P->r0, FIN_BI_QR0, false, g);
     launch_bicg_s(P->stream, C, P->sv, P->q, P->r, P->A, K > 0 ? P->zb[0] : nullptr, prm->omega,
-                  P->gpush[0], P->st);
-    if (K > 0) sz = krylov_jacobi(P, P->zb, P->sv, K, prm->omega, false, words, coef, launches);
-    krylov_matvec(P, sz, P->tv, P->sv, FIN_BI_TS, true, g);  // t_.s and t_.t
+                  F.g[0], P->st);
+    if (K > 0) sz = krylov_jacobi(P, F, P->zb, P->sv, K, prm->omega, false, words, coef, launches);
+    krylov_matvec(P, F, sz, P->tv, P->sv, FIN_BI_TS, true, g);  // t_.s and t_.t
     launch_bicg_update(P->stream, C, x, pz, sz, P->r, P->tv, P->sv, P->r0, P->kpart, P->st, c);
     launches += 5;
     // p, s (with their first Jacobi pass: z written, A read), two A*x (x, A, w,

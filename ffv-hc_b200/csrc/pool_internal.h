@@ -193,6 +193,7 @@ struct ffvgpu_pool {
   int act_next = 0;
   int grid_sweep = 0, grid_matvec = 0, grid_update = 0, grid_guides = 0, grid_mvpipe = 0;
   int grid_krylov = 0;  // the FP64 solvers' A*x and Jacobi passes
+  int grid_ring = 0;    // the same on the pipelined kernel
   int grid_cap = 0;  // test hook: at most this many CTAs per persistent grid (0: none)
   int grid_threads = 0;  // m_threads the grid sizes were computed for
 
