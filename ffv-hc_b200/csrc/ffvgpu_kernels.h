@@ -39,6 +39,14 @@ void launch_rbgs(cudaStream_t s, const KCtx& C, bool res, bool sweep, const doub
                  double* xout, const double* A, const double* b, RbgsGuides from,
                  const double* gin, double* gout, double omega, double* partials, SolveState* st,
                  int fin, int iter, bool pdl = false, const int32_t* order = nullptr);
+// The same pass with the coefficients through a ring of bulk copies
+// (rbgs_ring.cu): guides stored (gst) or, gst null, from the neighbours'
+// interiors.  pdl as above, after a pass of either kernel.
+void launch_rbgs_ring(cudaStream_t s, const KCtx& C, bool res, bool sweep, const double* xin,
+                      double* xout, const double* A, const double* b, const double* gst,
+                      double omega, double* partials, SolveState* st, int fin, int iter,
+                      bool pdl = false);
+int sm_count();  // of the current device
 // Each block's uniform record urec[blk][8] (Ap..At of cell 0, then 1.0 when
 // every cell has those seven coefficients, else 0.0), adding the uniform
 // blocks to *ucount.

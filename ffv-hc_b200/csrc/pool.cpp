@@ -207,6 +207,33 @@ ffvgpu_status read_ucount(ffvgpu_pool* P) {
   return FFVGPU_OK;
 }
 
+// Whether the FP64 stencil kernels of the pool are the ones that stream the
+// coefficients through a ring of bulk copies (rbgs_ring.cu, and the pipelined
+// kernel of the mixed form for A x and Jacobi passes): one CTA per SM that keeps
+// a varied block's 224 KB coming at HBM speed, but is the slower one where most
+// blocks are uniform; rbgs_block.cu and matvec_block.cu run two smaller CTAs per
+// SM that read coefficients as they use them.  us, two CTAs / ring, by the share
+// of blocks that are varied:
+//                  RBGS pass                         CG iteration, PreCount 2
+//    324 blocks    0.3 20/28   0.8 28/30   1 39/30     0.3  83/86    1  121/107
+//    548           0.5 37/40   0.65 48/41  1 53/44     0.5 140/134   1  188/162
+//   1164           0.3 71/71   0.4 78/72   1 121/81    0.4 244/231   1  364/281
+//   2366           0.3 119/122 0.4 136/124 1 242/142   0.3 403/383   1  682/507
+//   4692           0.3 213/239 0.4 248/244 1 485/293   0.3 741/720   1 1317/1003
+// (BiCGSTAB and the other PreCounts as CG), so the line lies at 35 % of the pool
+// and at more varied blocks than two per SM.
+ffvgpu_status ring_pool(ffvgpu_pool* P, bool* ring) {
+  ffvgpu_status s;
+  if ((s = ensure_urec(P))) return s;
+  *ring = false;
+  const int ctas = 2 * sm_count();
+  if (P->nb <= ctas) return FFVGPU_OK;
+  if ((s = read_ucount(P))) return s;
+  const int64_t varied = P->nb - P->ucount_h;
+  *ring = varied > ctas && 100 * varied > 35 * (int64_t)P->nb;
+  return FFVGPU_OK;
+}
+
 // The guide buffers that RBGS passes push into, for a neighbour table in which
 // every face is the other side's neighbour too (a shard's halo faces are not).
 ffvgpu_status ensure_push(ffvgpu_pool* P) {
@@ -271,37 +298,18 @@ MixCtx krylov_mix_ctx(const ffvgpu_pool* P, int fin) {
   return C;
 }
 
-// What a Krylov solve's A*x and Jacobi passes run on.  ring: the pipelined
-// kernel of the mixed form (one CTA per SM, coefficients through a ring of bulk
-// copies, guides from the neighbours' interiors); else matvec_block.cu (two
-// smaller CTAs per SM, which read coefficients as they use them, guides pushed
-// into g by the kernel that makes the operand).
+// What a Krylov solve's A*x and Jacobi passes run on (ring_pool): the pipelined
+// kernel, guides from the neighbours' interiors, or matvec_block.cu, guides
+// pushed into g by the kernel that makes the operand.
 struct KrylovForm {
   bool ring = false;
   int grid = 0;
   double* g[2] = {nullptr, nullptr};
 };
 
-// The ring keeps a varied block's 224 KB of coefficients streaming at HBM speed
-// (all 4692 blocks varied: A x 250 us a launch, a Jacobi pass 245; 238 at the
-// measured peak), but its one CTA per SM is the slower one where most blocks
-// are uniform.  us per CG iteration, PreCount 2, blocks /
-// ring, by the share of varied blocks:
-//    324 blocks: 0.3: 83 / 86,   0.8: 100 / 100,  1: 121 / 107
-//    548 blocks: 0.3: 128 / 127, 0.5: 140 / 134,  1: 188 / 162
-//   1164 blocks: 0.3: 225 / 222, 0.4: 244 / 231,  1: 364 / 281
-//   4692 blocks: 0.3: 741 / 720, 0.4: 824 / 770,  1: 1317 / 1003
-// so the line lies at a third of the pool and more varied blocks than
-// matvec_block.cu has CTAs (BiCGSTAB and the other PreCounts agree).
 ffvgpu_status krylov_form(ffvgpu_pool* P, KrylovForm* F) {
   ffvgpu_status s;
-  if ((s = ensure_kpipe(P))) return s;
-  if (!P->grid_krylov) P->grid_krylov = matvec_block_grid();
-  if (P->nb > P->grid_krylov) {
-    if ((s = read_ucount(P))) return s;
-    const int64_t varied = P->nb - P->ucount_h;
-    F->ring = varied > P->grid_krylov && 100 * varied > 35 * (int64_t)P->nb;
-  }
+  if ((s = ring_pool(P, &F->ring)) || (s = ensure_kpipe(P))) return s;
   if (F->ring) {
     if (!P->grid_ring) {
       int a, b, c, d;
@@ -309,6 +317,7 @@ ffvgpu_status krylov_form(ffvgpu_pool* P, KrylovForm* F) {
     }
     F->grid = P->grid_ring;
   } else {
+    if (!P->grid_krylov) P->grid_krylov = matvec_block_grid();
     F->grid = P->grid_krylov;
     if ((s = ensure_push(P))) return s;
     F->g[0] = P->gpush[0];
@@ -349,6 +358,19 @@ double* krylov_jacobi(ffvgpu_pool* P, const KrylovForm& F, double* const z[2], c
     launches++;
   }
   return z[(K - 1) & 1];
+}
+
+// One RBGS pass over the C.nb first blocks, on the ring or not.
+void rbgs_pass(ffvgpu_pool* P, bool ring, const KCtx& C, bool res, bool sweep, const double* xin,
+               double* xout, RbgsGuides from, const double* gin, double* gout, double omega,
+               int fin, int iter, bool pdl = false, const int32_t* order = nullptr) {
+  if (ring)
+    launch_rbgs_ring(P->stream, C, res, sweep, xin, xout, P->A, P->b,
+                     from == RbgsGuides::STORED ? gin : nullptr, omega, P->partials, P->st, fin,
+                     iter, pdl);
+  else
+    launch_rbgs(P->stream, C, res, sweep, xin, xout, P->A, P->b, from, gin, gout, omega,
+                P->partials, P->st, fin, iter, pdl, order);
 }
 
 // Derives the neighbour table from levels and block indices.
@@ -889,9 +911,10 @@ ffvgpu_status ffvgpu_calc_r2(ffvgpu_pool* P, double* rr) {
   ffvgpu_status s;
   if ((s = require_system(P))) return s;
   if ((s = reset_state(P, 0.0, 0, nullptr))) return s;
-  if ((s = ensure_urec(P))) return s;
-  launch_rbgs(P->stream, P->ctx(P->bc_p), true, false, P->x[P->xcur], nullptr, P->A, P->b,
-              RbgsGuides::STORED, P->gx, nullptr, 0.0, P->partials, P->st, FIN_STORE, 0);
+  bool ring;
+  if ((s = ring_pool(P, &ring))) return s;
+  rbgs_pass(P, ring, P->ctx(P->bc_p), true, false, P->x[P->xcur], nullptr, RbgsGuides::STORED,
+            P->gx, nullptr, 0.0, FIN_STORE, 0);
   CK(cudaGetLastError());
   SolveState h;
   if ((s = read_state(P, &h))) return s;
@@ -910,10 +933,10 @@ ffvgpu_status ffvgpu_rbgs_sweep(ffvgpu_pool* P, double omega) {
   ffvgpu_status s;
   if ((s = require_system(P))) return s;
   if ((s = reset_state(P, 0.0, 0, nullptr))) return s;
-  if ((s = ensure_urec(P))) return s;
-  launch_rbgs(P->stream, P->ctx(P->bc_p), false, true, P->x[P->xcur], P->x[1 - P->xcur],
-              P->A, P->b, RbgsGuides::STORED, P->gx, nullptr, omega, P->partials, P->st,
-              FIN_STORE, 0);
+  bool ring;
+  if ((s = ring_pool(P, &ring))) return s;
+  rbgs_pass(P, ring, P->ctx(P->bc_p), false, true, P->x[P->xcur], P->x[1 - P->xcur],
+            RbgsGuides::STORED, P->gx, nullptr, omega, FIN_STORE, 0);
   P->xcur = 1 - P->xcur;
   launch_exchange(P->stream, P->ctx(P->bc_p), P->x[P->xcur], P->gx);
   CK(cudaGetLastError());
@@ -946,12 +969,18 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
     return FFVGPU_OK;
   }
   if ((s = ensure_hist(P, N))) return s;
-  if ((s = ensure_urec(P))) return s;
+  bool ring;
+  if ((s = ring_pool(P, &ring))) return s;
   if ((s = reset_state(P, prm->epsilon, N, P->hist_d))) return s;
-  if ((s = ensure_push(P))) return s;
-  const RbgsGuides from = P->gpush[0] ? RbgsGuides::PUSHED : RbgsGuides::PULL;
-  if ((s = ensure_kpipe(P))) return s;
-  const int32_t* order = P->kpipe + 1;
+  RbgsGuides from = RbgsGuides::PULL;
+  double* g[2] = {nullptr, nullptr};
+  const int32_t* order = nullptr;
+  if (!ring) {
+    if ((s = ensure_push(P)) || (s = ensure_kpipe(P))) return s;
+    for (int k = 0; k < 2; ++k) g[k] = P->gpush[k];
+    if (g[0]) from = RbgsGuides::PUSHED;
+    order = P->kpipe + 1;
+  }
   const KCtx C = P->ctx(P->bc_p);
   const int every = prm->check_every > 0 ? prm->check_every : 32;
   const bool poll = prm->epsilon > 0.0;
@@ -959,9 +988,8 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   launch_dot(P->stream, C, P->b, P->b, P->partials, P->st, FIN_BB, 0);
   int launches = 1;
   const int c0 = P->xcur;
-  launch_rbgs(P->stream, C, false, true, P->x[c0], P->x[1 - c0], P->A, P->b,
-              RbgsGuides::STORED, P->gx, P->gpush[0], prm->omega, P->partials, P->st, FIN_RBGS, 0,
-              false, order);
+  rbgs_pass(P, ring, C, false, true, P->x[c0], P->x[1 - c0], RbgsGuides::STORED, P->gx, g[0],
+            prm->omega, FIN_RBGS, 0, false, order);
   launches++;
   CK(cudaEventRecord(P->ev2, P->stream));
   int swept = 0;
@@ -970,9 +998,8 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   // poll or a timing event sits between them.
   bool polled_last = true;
   for (int n = 2; n <= N; ++n) {
-    launch_rbgs(P->stream, C, true, true, P->x[(c0 + n - 1) & 1], P->x[(c0 + n) & 1], P->A, P->b,
-                from, P->gpush[n & 1], P->gpush[(n + 1) & 1], prm->omega, P->partials, P->st,
-                FIN_RBGS, n - 1, !polled_last, order);
+    rbgs_pass(P, ring, C, true, true, P->x[(c0 + n - 1) & 1], P->x[(c0 + n) & 1], from, g[n & 1],
+              g[(n + 1) & 1], prm->omega, FIN_RBGS, n - 1, !polled_last, order);
     polled_last = false;
     swept++;
     launches++;
@@ -984,9 +1011,8 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
     }
   }
   CK(cudaEventRecord(P->ev3, P->stream));
-  launch_rbgs(P->stream, C, true, false, P->x[(c0 + N) & 1], nullptr, P->A, P->b,
-              from, P->gpush[(N + 1) & 1], nullptr, prm->omega, P->partials, P->st, FIN_RBGS, N,
-              false, order);
+  rbgs_pass(P, ring, C, true, false, P->x[(c0 + N) & 1], nullptr, from, g[(N + 1) & 1], nullptr,
+            prm->omega, FIN_RBGS, N, false, order);
   launches++;
   CK(cudaEventRecord(P->ev1, P->stream));
   CK(cudaGetLastError());
@@ -1044,7 +1070,8 @@ ffvgpu_status ffvgpu_solve_rbgs_fixed_average(ffvgpu_pool* P, const ffvgpu_iter_
     if (res) *res = R;
     return FFVGPU_OK;
   }
-  if ((s = ensure_hist(P, N)) || (s = ensure_urec(P))) return s;
+  bool ring;
+  if ((s = ensure_hist(P, N)) || (s = ring_pool(P, &ring))) return s;
   SolveState h0;
   std::memset(&h0, 0, sizeof(h0));
   h0.eps = prm->epsilon;
@@ -1065,14 +1092,14 @@ ffvgpu_status ffvgpu_solve_rbgs_fixed_average(ffvgpu_pool* P, const ffvgpu_iter_
   for (int n = 1; n <= N; ++n) {
     // once the solve has stopped these kernels return at entry: the iterate
     // kept is the one of the stopping iteration (below)
-    launch_rbgs(P->stream, C, false, true, P->x[cur], P->x[1 - cur], P->A, P->b,
-                n == 1 ? RbgsGuides::STORED : RbgsGuides::PULL, n == 1 ? P->gx : nullptr, nullptr,
-                prm->omega, P->partials, P->st, FIN_STORE, n);
+    rbgs_pass(P, ring, C, false, true, P->x[cur], P->x[1 - cur],
+              n == 1 ? RbgsGuides::STORED : RbgsGuides::PULL, n == 1 ? P->gx : nullptr, nullptr,
+              prm->omega, FIN_STORE, n);
     cur = 1 - cur;
     launch_sum(P->stream, C, P->x[cur], P->partials, P->st, FIN_FA_SHIFT);
     launch_shift(P->stream, C, P->x[cur], P->st);
-    launch_rbgs(P->stream, C, true, false, P->x[cur], nullptr, P->A, P->b,
-                RbgsGuides::PULL, nullptr, nullptr, prm->omega, P->partials, P->st, FIN_RBGS, n);
+    rbgs_pass(P, ring, C, true, false, P->x[cur], nullptr, RbgsGuides::PULL, nullptr, nullptr,
+              prm->omega, FIN_RBGS, n);
     launches += 4;
     passes++;
     if (poll && (n % every) == 0) {
@@ -1351,13 +1378,15 @@ ffvgpu_status ffvgpu_rbgs_pass(ffvgpu_pool* P, int32_t blocks, int32_t residual,
   cudaSetDevice(P->device);
   ffvgpu_status s;
   if ((s = require_system(P))) return s;
-  if ((s = ensure_urec(P))) return s;
+  bool ring;
+  if ((s = ring_pool(P, &ring))) return s;
   if ((s = reset_state(P, 0.0, 0, nullptr))) return s;
   KCtx C = P->ctx(P->bc_p);
   C.nb = blocks;
   const int c = P->xcur;
-  launch_rbgs(P->stream, C, res, swp, P->x[c], swp ? P->x[1 - c] : nullptr, P->A, P->b,
-              st ? RbgsGuides::STORED : RbgsGuides::PULL, st ? P->gx : nullptr, nullptr, omega, P->partials, P->st, FIN_STORE, 0);
+  rbgs_pass(P, ring, C, res, swp, P->x[c], swp ? P->x[1 - c] : nullptr,
+            st ? RbgsGuides::STORED : RbgsGuides::PULL, st ? P->gx : nullptr, nullptr, omega,
+            FIN_STORE, 0);
   CK(cudaGetLastError());
   if (swp) P->xcur = 1 - c;
   SolveState h;

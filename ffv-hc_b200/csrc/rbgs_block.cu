@@ -325,18 +325,6 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
   }
 }
 
-int sm_count() {
-  static std::mutex mu;
-  static int count[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  int local = 0;
-  int& n = dev >= 0 && dev < 64 ? count[dev] : local;
-  if (n == 0) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n > 0 ? n : 1;
-}
-
 template <bool R, bool W, int G>
 void launch_one(cudaStream_t s, const KCtx& C, const double* xin, double* xout, const double* A,
                 const double* b, const double* gst, double* gout, double omega, double* partials,
@@ -348,15 +336,29 @@ void launch_one(cudaStream_t s, const KCtx& C, const double* xin, double* xout, 
   const int grid = std::min(C.nb, 2 * sms);
   auto kernel = one ? rbgs_block_kernel<R, W, G, 1> : rbgs_block_kernel<R, W, G, 2>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
-  // With up to eight blocks per SM the varied blocks, which take three times as
-  // long, go first so that none is left for the end (324 blocks: 26 us a pass,
-  // 30 in block order); with more the order mixes them, so that one CTA's
-  // coefficient loads overlap the other's arithmetic (4692: 151 us, 159).
+  // With up to twelve blocks per SM the varied blocks, which take three times as
+  // long, go first so that none is left for the end; with more the order mixes
+  // them, so that one CTA's coefficient loads overlap the other's arithmetic.
+  // us per pass, varied first / block order, by blocks per SM: 2.2: 24.0 / 29.0,
+  // 3.7: 34.4 / 35.8, 4.8: 45.8 / 53.7, 7.9: 59.5 / 68.6, 11.3: 74.5 / 77.9,
+  // 15.3: 107.6 / 106.2, 21: 108.2 / 105.5, 32: 158.4 / 147.9.
   launch_dep(kernel, grid, NT, sizeof(Smem), s, pdl, C, xin, xout, A, b, gst, gout, omega,
-             partials, st, fin, iter, C.nb <= 8 * sms ? order : nullptr);
+             partials, st, fin, iter, C.nb <= 12 * sms ? order : nullptr);
 }
 
 }  // namespace
+
+int sm_count() {
+  static std::mutex mu;
+  static int count[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  int local = 0;
+  int& n = dev >= 0 && dev < 64 ? count[dev] : local;
+  if (n == 0) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n > 0 ? n : 1;
+}
 
 void launch_rbgs(cudaStream_t s, const KCtx& C, bool res, bool sweep, const double* xin,
                  double* xout, const double* A, const double* b, RbgsGuides from,

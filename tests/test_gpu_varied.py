@@ -6,6 +6,7 @@ an upload of A moves a pool from one side to the other."""
 import numpy as np
 import pytest
 
+import ffvgpu
 from helpers import VC, assert_bitwise, device_problem, interior, problem
 
 pytestmark = pytest.mark.gpu
@@ -51,7 +52,47 @@ def test_krylov_on_varied_pools(root, share, solver, args):
     O.close()
 
 
-@pytest.mark.parametrize("solver,args", [("cg", (1.0, 2, 4, 0.0)), ("bicgstab", (1.0, 2, 4, 0.0))])
+@pytest.mark.parametrize("root,share", [((9, 6, 6), 1.0), ((37, 4, 2), 1.0), ((11, 9, 3), 1.0),
+                                        ((9, 6, 6), 0.95), ((10, 9, 9), 0.5), ((10, 9, 9), 0.3)])
+@pytest.mark.parametrize("solver,args", [("rbgs", (1.1, 1, 0.0)), ("rbgs", (1.1, 6, 0.0)),
+                                         ("rbgs_fixed_average", (1.0, None, 3, 0.0))])
+def test_rbgs_on_varied_pools(root, share, solver, args):
+    g, inp, O = problem(0, root_grid=root, radius=0.5)
+    P = device_problem(g, inp)
+    set_varied(g, P, O, share)
+    run(g, P, O, solver, args)
+    P.close()
+    O.close()
+
+
+def test_single_rbgs_calls_on_a_varied_pool():
+    """Stored guides as uploaded, then as the sweep's exchange left them; the early stop of a
+    solve with a criterion; a wait limit of 0 ends in TIMEOUT and leaves the pool usable."""
+    g, inp, O = problem(3)
+    P = device_problem(g, inp)
+    set_varied(g, P, O, 0.9)
+    x = np.random.default_rng(4).standard_normal((g.nb, 20, 20, 20))
+    P.upload("X", x, VC)
+    O.field("X")[...] = x
+    for _ in range(2):
+        assert P.calc_r2() == O.calc_r2()
+        P.rbgs_sweep(1.2)
+        O.rbgs_sweep(1.2)
+        O.exchange("X", ffvgpu.P_BC_TYPE, ffvgpu.P_BC_VALUE)
+        assert_bitwise(interior(P.download("X", VC)), interior(O.field("X")), "x")
+    run(g, P, O, "rbgs", (1.2, 200, 0.02))
+    P.set_wait_limit(0.0)
+    with pytest.raises(ffvgpu.FFVGPUError) as e:
+        P.solve_rbgs(1.2, 5, 0.0)
+    assert e.value.status == ffvgpu.TIMEOUT and "drain" not in str(e.value)
+    P.set_wait_limit(4.0)
+    run(g, P, O, "rbgs", (1.2, 5, 0.0))
+    P.close()
+    O.close()
+
+
+@pytest.mark.parametrize("solver,args", [("cg", (1.0, 2, 4, 0.0)), ("bicgstab", (1.0, 2, 4, 0.0)),
+                                         ("rbgs", (1.0, 7, 0.0))])
 def test_coefficients_replaced_between_solves(solver, args):
     """2:1 faces (level 3), A replaced between solves so that the pool changes sides twice, and
     grids capped to one CTA."""
