@@ -21,6 +21,8 @@ struct KCtx {
   int nb;
   int first;
   uint64_t wait_ns;    // limit of every bounded device wait (ffvgpu_pool_set_wait_limit)
+  // test hook of the RBGS kernels: copies that a pass then waits for are not issued
+  int stall;
   // [blocks][8] uniform records of A (launch_urec), or
   // null: every block streams all its coefficients
   const double* urec;

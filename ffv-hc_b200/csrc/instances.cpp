@@ -851,9 +851,9 @@ ffvgpu_status ffvgpu_mixed_poll(ffvgpu_pool* P, int32_t* finished, int32_t capac
   return FFVGPU_OK;
 }
 
-// Test hook: the next mixed solve's sweep kernel waits for a copy it never
-// issues, so the wait runs out after the pool's wait limit and the solve ends
-// with FFVGPU_TIMEOUT; nothing is in flight, so nothing is drained.
+// Test hook: the next mixed or RBGS solve's sweep kernel waits for a copy it
+// never issues, so the wait runs out after the pool's wait limit and the solve
+// ends with FFVGPU_TIMEOUT; that copy is not waited for on the way out.
 ffvgpu_status ffvgpu_pool_stall_next_solve(ffvgpu_pool* P) {
   if (!P) return bad("null pool");
   P->stall_sweep = 1;

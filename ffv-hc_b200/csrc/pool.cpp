@@ -981,7 +981,11 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
     if (g[0]) from = RbgsGuides::PUSHED;
     order = P->kpipe + 1;
   }
-  const KCtx C = P->ctx(P->bc_p);
+  KCtx C = P->ctx(P->bc_p);
+  if (P->stall_sweep == 1) {  // the test hook covers one solve
+    C.stall = 1;
+    P->stall_sweep = 0;
+  }
   const int every = prm->check_every > 0 ? prm->check_every : 32;
   const bool poll = prm->epsilon > 0.0;
   CK(cudaEventRecord(P->ev0, P->stream));

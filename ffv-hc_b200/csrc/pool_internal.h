@@ -180,8 +180,8 @@ struct ffvgpu_pool {
   int mgraph_cf = 0;
   int mgraph_d64 = 0;
   int mgraph_depth = 0, mgraph_threads = 0, mgraph_sweep_threads = 0, mgraph_mvform = -1;
-  int stall_sweep = 0;  // test hook: 1 sweep, 2 A*x (ffvgpu_pool_stall_next_solve / _matvec),
-                        // cleared when a solve ends
+  int stall_sweep = 0;  // test hook: 1 mixed sweep or RBGS pass, 2 A*x
+                        // (ffvgpu_pool_stall_next_solve / _matvec), for one solve
   int64_t m_launches = 0;
   int64_t m_bytes = 0;
   // active-block list of the persistent kernels: device [1 + capacity]
@@ -205,6 +205,7 @@ struct ffvgpu_pool {
     C.nb = nb;
     C.first = 0;
     C.wait_ns = wait_ns;
+    C.stall = 0;
     C.urec = (urec && urec_version == sys_version) ? urec : nullptr;
     return C;
   }

@@ -210,8 +210,11 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
     if (b >= 0 && tid < REC_THREADS)
       fetch_record(S.rec[m % 3], &S.rbar[m % 3], C.nbr, C.urec, b);
   };
+  // test hook (KCtx::stall): no b for a CTA's third block, its second where no
+  // CTA has three, its only one where none has two
+  const int stall_at = C.stall ? (nb > 2 * grid ? 2 : nb > grid ? 1 : 0) : -1;
   auto fetch_b = [&](int b, int m) {  // b of the CTA's m-th block
-    if (b >= 0 && tid == 32) {
+    if (b >= 0 && tid == 32 && m != stall_at) {
       async::mbar_expect_tx(&S.bbar[m & 1], BLOCK_CELLS * 8);
       async::bulk_g2s(S.b[m & 1], bvec + (size_t)b * BLOCK_CELLS, BLOCK_CELLS * 8, &S.bbar[m & 1]);
     }
@@ -227,8 +230,8 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
   fetch_rec(blk, 0);
   fetch_b(blk, 0);
   fetch_rec(next, 1);
-  // with a limit of 0 nothing is waited for, and the first record has only
-  // just been asked for
+  // a limit of 0 lets nothing be waited for: the pass gives up here, whether or
+  // not the record happens to have landed by the time a wait would look
   bool ok = blk < 0 || C.wait_ns != 0;
   std::conditional_t<PER_SM == 1, Held, Varied> AV{A + (size_t)blk * 7 * BLOCK_CELLS + slot(tid)};
   pdl_release();
@@ -296,7 +299,7 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
     // block n's and n + 1's records and block n's b (a step issues the ones
     // after them only once its waits have succeeded).
     if (tid == 0) {
-      bool drained = async::mbar_drain(&S.bbar[n & 1], (n >> 1) & 1);
+      bool drained = n == stall_at || async::mbar_drain(&S.bbar[n & 1], (n >> 1) & 1);
       drained = async::mbar_drain(&S.rbar[n % 3], (n / 3) & 1) && drained;
       if (next >= 0) drained = async::mbar_drain(&S.rbar[(n + 1) % 3], ((n + 1) / 3) & 1) && drained;
       if (!ok) {

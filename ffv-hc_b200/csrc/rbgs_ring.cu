@@ -151,7 +151,9 @@ rbgs_ring_kernel(const __grid_constant__ KCtx C, const double* xin, double* __re
   }
   __syncthreads();
   const int myblocks = (blockIdx.x < nb) ? (nb - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  const int total_slots = myblocks * SLOTS;
+  // (test hook KCtx::stall: the producer issues nothing, so the consumers' first
+  // wait runs out)
+  const int total_slots = C.stall ? 0 : myblocks * SLOTS;
   // is this CTA's m-th block uniform
   auto uniform = [&](int m) {
     return m < 32 * UMASK_WORDS && ((S.umask[m >> 5] >> (m & 31)) & 1u);
@@ -192,7 +194,7 @@ rbgs_ring_kernel(const __grid_constant__ KCtx C, const double* xin, double* __re
       for (; g < (uint32_t)STAGES && g < (uint32_t)total_slots; ++g) issue_slot(g);
       tile::pdl_wait();
       const bool skip = *((volatile const int32_t*)&st->done) != 0;
-      if (!skip && myblocks > 0) {
+      if (!skip && total_slots > 0) {
         ++nx[0];
         issue_x(0, 0);
       }

@@ -586,7 +586,7 @@ class Pool:
         _check(lib().ffvgpu_pool_set_wait_limit(self._h, float(seconds)), "pool_set_wait_limit")
 
     def stall_next_solve(self):
-        """Test hook: the next mixed solve's sweep waits for a copy never issued."""
+        """Test hook: the next mixed or RBGS solve's sweep waits for a copy never issued."""
         _check(lib().ffvgpu_pool_stall_next_solve(self._h), "pool_stall_next_solve")
 
     def cap_grids(self, ctas):

@@ -143,9 +143,9 @@ ffvgpu_status ffvgpu_pool_set_stream(ffvgpu_pool* pool, void* stream);
  * counterpart is the MPI runtime's own timeouts. */
 ffvgpu_status ffvgpu_pool_set_wait_limit(ffvgpu_pool* pool, double seconds);
 /* Test hook for the timeout path (no counterpart in the reference): the next
- * mixed-form solve on the pool waits in its sweep kernel for a copy that is
- * never issued, so that wait runs out after the wait limit and the solve ends
- * with FFVGPU_TIMEOUT.  The hook covers that one solve. */
+ * mixed-form or RBGS solve on the pool waits in its sweep kernel for a copy
+ * that is never issued, so that wait runs out after the wait limit and the
+ * solve ends with FFVGPU_TIMEOUT.  The hook covers that one solve. */
 ffvgpu_status ffvgpu_pool_stall_next_solve(ffvgpu_pool* pool);
 /* The same for the pipelined A*x kernel (matvec_form 0): its producer issues
  * no copy, so the consumers' first wait for a slot runs out. */
