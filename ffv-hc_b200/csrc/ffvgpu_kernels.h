@@ -21,8 +21,6 @@ struct KCtx {
   int nb;
   int first;
   uint64_t wait_ns;    // limit of every bounded device wait (ffvgpu_pool_set_wait_limit)
-  // test hook of the RBGS kernels: copies that a pass then waits for are not issued
-  int stall;
   // [blocks][8] uniform records of A (launch_urec), or
   // null: every block streams all its coefficients
   const double* urec;
@@ -41,13 +39,20 @@ void launch_rbgs(cudaStream_t s, const KCtx& C, bool res, bool sweep, const doub
                  double* xout, const double* A, const double* b, RbgsGuides from,
                  const double* gin, double* gout, double omega, double* partials, SolveState* st,
                  int fin, int iter, bool pdl = false, const int32_t* order = nullptr);
+// Test hook: the first sweep (stored guides, no residual), in the form that
+// launch_rbgs or, ring, launch_rbgs_ring would take, with copies left out that
+// it then waits for.
+void launch_rbgs_stalled(cudaStream_t s, const KCtx& C, bool ring, const double* xin,
+                         double* xout, const double* A, const double* b, const double* gin,
+                         double* gout, double omega, double* partials, SolveState* st,
+                         const int32_t* order);
 // The same pass with the coefficients through a ring of bulk copies
 // (rbgs_ring.cu): guides stored (gst) or, gst null, from the neighbours'
 // interiors.  pdl as above, after a pass of either kernel.
 void launch_rbgs_ring(cudaStream_t s, const KCtx& C, bool res, bool sweep, const double* xin,
                       double* xout, const double* A, const double* b, const double* gst,
                       double omega, double* partials, SolveState* st, int fin, int iter,
-                      bool pdl = false);
+                      bool pdl = false, bool stall = false);
 int sm_count();  // of the current device
 // Each block's uniform record urec[blk][8] (Ap..At of cell 0, then 1.0 when
 // every cell has those seven coefficients, else 0.0), adding the uniform

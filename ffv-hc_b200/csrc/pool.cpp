@@ -981,19 +981,21 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
     if (g[0]) from = RbgsGuides::PUSHED;
     order = P->kpipe + 1;
   }
-  KCtx C = P->ctx(P->bc_p);
-  if (P->stall_sweep == 1) {  // the test hook covers one solve
-    C.stall = 1;
-    P->stall_sweep = 0;
-  }
+  const KCtx C = P->ctx(P->bc_p);
   const int every = prm->check_every > 0 ? prm->check_every : 32;
   const bool poll = prm->epsilon > 0.0;
   CK(cudaEventRecord(P->ev0, P->stream));
   launch_dot(P->stream, C, P->b, P->b, P->partials, P->st, FIN_BB, 0);
   int launches = 1;
   const int c0 = P->xcur;
-  rbgs_pass(P, ring, C, false, true, P->x[c0], P->x[1 - c0], RbgsGuides::STORED, P->gx, g[0],
-            prm->omega, FIN_RBGS, 0, false, order);
+  if (P->stall_sweep == 1) {  // the test hook covers one solve
+    P->stall_sweep = 0;
+    launch_rbgs_stalled(P->stream, C, ring, P->x[c0], P->x[1 - c0], P->A, P->b, P->gx, g[0],
+                        prm->omega, P->partials, P->st, order);
+  } else {
+    rbgs_pass(P, ring, C, false, true, P->x[c0], P->x[1 - c0], RbgsGuides::STORED, P->gx, g[0],
+              prm->omega, FIN_RBGS, 0, false, order);
+  }
   launches++;
   CK(cudaEventRecord(P->ev2, P->stream));
   int swept = 0;

@@ -205,7 +205,6 @@ struct ffvgpu_pool {
     C.nb = nb;
     C.first = 0;
     C.wait_ns = wait_ns;
-    C.stall = 0;
     C.urec = (urec && urec_version == sys_version) ? urec : nullptr;
     return C;
   }

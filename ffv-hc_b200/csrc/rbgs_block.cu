@@ -186,7 +186,9 @@ struct __align__(128) Smem {
 };
 static_assert(2 * (sizeof(Smem) + 1024) <= 228 * 1024, "two CTAs per SM");
 
-template <bool RES, bool SWEEP, int SRC, int PER_SM>
+// STALL (test hook): no b for a CTA's third block, its second where no CTA has
+// three, its only one where none has two.
+template <bool RES, bool SWEEP, int SRC, int PER_SM, bool STALL>
 __global__ void __launch_bounds__(NT, PER_SM)
 rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
                   double* __restrict__ xout, const double* __restrict__ A,
@@ -210,11 +212,9 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
     if (b >= 0 && tid < REC_THREADS)
       fetch_record(S.rec[m % 3], &S.rbar[m % 3], C.nbr, C.urec, b);
   };
-  // test hook (KCtx::stall): no b for a CTA's third block, its second where no
-  // CTA has three, its only one where none has two
-  const int stall_at = C.stall ? (nb > 2 * grid ? 2 : nb > grid ? 1 : 0) : -1;
+  auto stalled = [&](int m) { return STALL && m == (nb > 2 * grid ? 2 : nb > grid ? 1 : 0); };
   auto fetch_b = [&](int b, int m) {  // b of the CTA's m-th block
-    if (b >= 0 && tid == 32 && m != stall_at) {
+    if (b >= 0 && tid == 32 && !stalled(m)) {
       async::mbar_expect_tx(&S.bbar[m & 1], BLOCK_CELLS * 8);
       async::bulk_g2s(S.b[m & 1], bvec + (size_t)b * BLOCK_CELLS, BLOCK_CELLS * 8, &S.bbar[m & 1]);
     }
@@ -299,7 +299,7 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
     // block n's and n + 1's records and block n's b (a step issues the ones
     // after them only once its waits have succeeded).
     if (tid == 0) {
-      bool drained = n == stall_at || async::mbar_drain(&S.bbar[n & 1], (n >> 1) & 1);
+      bool drained = stalled(n) || async::mbar_drain(&S.bbar[n & 1], (n >> 1) & 1);
       drained = async::mbar_drain(&S.rbar[n % 3], (n / 3) & 1) && drained;
       if (next >= 0) drained = async::mbar_drain(&S.rbar[(n + 1) % 3], ((n + 1) / 3) & 1) && drained;
       if (!ok) {
@@ -328,7 +328,7 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
   }
 }
 
-template <bool R, bool W, int G>
+template <bool R, bool W, int G, bool STALL = false>
 void launch_one(cudaStream_t s, const KCtx& C, const double* xin, double* xout, const double* A,
                 const double* b, const double* gst, double* gout, double omega, double* partials,
                 SolveState* st, int fin, int iter, bool pdl, const int32_t* order) {
@@ -337,7 +337,7 @@ void launch_one(cudaStream_t s, const KCtx& C, const double* xin, double* xout, 
   // block's colour-1 coefficients instead (72 blocks: 13.7 us a pass, 16.8)
   const bool one = C.nb <= sms;
   const int grid = std::min(C.nb, 2 * sms);
-  auto kernel = one ? rbgs_block_kernel<R, W, G, 1> : rbgs_block_kernel<R, W, G, 2>;
+  auto kernel = one ? rbgs_block_kernel<R, W, G, 1, STALL> : rbgs_block_kernel<R, W, G, 2, STALL>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
   // With up to twelve blocks per SM the varied blocks, which take three times as
   // long, go first so that none is left for the end; with more the order mixes
@@ -361,6 +361,18 @@ int sm_count() {
   int& n = dev >= 0 && dev < 64 ? count[dev] : local;
   if (n == 0) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
   return n > 0 ? n : 1;
+}
+
+void launch_rbgs_stalled(cudaStream_t s, const KCtx& C, bool ring, const double* xin,
+                         double* xout, const double* A, const double* b, const double* gin,
+                         double* gout, double omega, double* partials, SolveState* st,
+                         const int32_t* order) {
+  if (ring)
+    launch_rbgs_ring(s, C, false, true, xin, xout, A, b, gin, omega, partials, st, FIN_RBGS, 0,
+                     false, true);
+  else
+    launch_one<false, true, tile::STORED, true>(s, C, xin, xout, A, b, gin, gout, omega, partials,
+                                                st, FIN_RBGS, 0, false, order);
 }
 
 void launch_rbgs(cudaStream_t s, const KCtx& C, bool res, bool sweep, const double* xin,

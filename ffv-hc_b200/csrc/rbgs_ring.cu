@@ -110,7 +110,9 @@ __device__ __forceinline__ void consumer_sync() {
 
 }  // namespace pipe
 
-template <bool DO_RES, bool DO_SWEEP>
+// STALL (test hook): the producer issues nothing, so the consumers' first wait
+// runs out.
+template <bool DO_RES, bool DO_SWEEP, bool STALL>
 __global__ void __launch_bounds__(pipe::NTHREADS, 1)
 rbgs_ring_kernel(const __grid_constant__ KCtx C, const double* xin, double* __restrict__ xout,
                  const double* __restrict__ A, const double* __restrict__ bvec, const double* gst,
@@ -151,9 +153,7 @@ rbgs_ring_kernel(const __grid_constant__ KCtx C, const double* xin, double* __re
   }
   __syncthreads();
   const int myblocks = (blockIdx.x < nb) ? (nb - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  // (test hook KCtx::stall: the producer issues nothing, so the consumers' first
-  // wait runs out)
-  const int total_slots = C.stall ? 0 : myblocks * SLOTS;
+  const int total_slots = STALL ? 0 : myblocks * SLOTS;
   // is this CTA's m-th block uniform
   auto uniform = [&](int m) {
     return m < 32 * UMASK_WORDS && ((S.umask[m >> 5] >> (m & 31)) & 1u);
@@ -420,22 +420,24 @@ rbgs_ring_kernel(const __grid_constant__ KCtx C, const double* xin, double* __re
 }
 
 namespace {
-template <bool R, bool W>
+template <bool R, bool W, bool STALL = false>
 void launch_one(cudaStream_t s, const KCtx& C, const double* xin, double* xout, const double* A,
                 const double* b, const double* gst, double omega, double* partials,
                 SolveState* st, int fin, int iter, bool pdl) {
-  cudaFuncSetAttribute(rbgs_ring_kernel<R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const auto kernel = rbgs_ring_kernel<R, W, STALL>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(pipe::Smem));
-  launch_dep(rbgs_ring_kernel<R, W>, std::min(C.nb, sm_count()), pipe::NTHREADS,
-             sizeof(pipe::Smem), s, pdl, C, xin, xout, A, b, gst, omega, partials, st, fin, iter);
+  launch_dep(kernel, std::min(C.nb, sm_count()), pipe::NTHREADS, sizeof(pipe::Smem), s, pdl, C,
+             xin, xout, A, b, gst, omega, partials, st, fin, iter);
 }
 }  // namespace
 
 void launch_rbgs_ring(cudaStream_t s, const KCtx& C, bool res, bool sweep, const double* xin,
                       double* xout, const double* A, const double* b, const double* gst,
                       double omega, double* partials, SolveState* st, int fin, int iter,
-                      bool pdl) {
-  const auto launch = res && sweep ? launch_one<true, true>
+                      bool pdl, bool stall) {
+  const auto launch = stall          ? launch_one<false, true, true>
+                      : res && sweep ? launch_one<true, true>
                       : sweep      ? launch_one<false, true>
                                    : launch_one<true, false>;
   launch(s, C, xin, xout, A, b, gst, omega, partials, st, fin, iter, pdl);
