@@ -27,8 +27,8 @@ struct MixCtx {
   int capacity;
   int first;
   uint64_t wait_ns;    // limit of every bounded device wait (ffvgpu_pool_set_wait_limit)
-  int stall;           // test hook: 1 the sweep kernel, 2 the pipelined A*x issues no copy,
-                       // so its first wait runs out
+  int stall;           // test hook: a copy is not issued, so that the wait for it runs out:
+                       // 1 the sweep kernel, 2 A*x and the FP64 solvers' Jacobi passes
   int cf;              // coarse-fine flux correction in the FP64 residual and A*x
   int depth;           // sweep kernel: L2 prefetch distance in blocks (staging depth, >= 1)
   int sweep_threads;   // sweep kernel: 256 (two rows per thread, the default) or 512 (one row)

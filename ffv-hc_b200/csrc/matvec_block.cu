@@ -33,7 +33,7 @@ namespace {
 
 using namespace tile;
 
-constexpr int ROLE_MATVEC = 32;  // SolveState::timeout_where bit
+constexpr int ROLE_MATVEC = 64;  // SolveState::timeout_where bit of this kernel's waits
 constexpr int CAP = NT;          // list entries per chunk
 
 struct __align__(128) Smem {
@@ -134,7 +134,8 @@ __device__ __forceinline__ void cells(const double* T, double (&X)[2][NC], const
     for (int n = 0; n < NC; ++n) X[0][n] = Y0[JAC ? n : 0];
 }
 
-template <int NV, bool JAC, int SRC>
+// STALL (test hook): no w0 for the last block of the CTAs with most.
+template <int NV, bool JAC, int SRC, bool STALL>
 __global__ void __launch_bounds__(NT, 2)
 matvec_block_kernel(const __grid_constant__ MixCtx C, const double* __restrict__ x,
                     const double* __restrict__ A, double* __restrict__ y,
@@ -155,8 +156,9 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const double* __restrict__
     if (tid < REC_THREADS)
       fetch_record(S.rec[m % 3], &S.rbar[m % 3], C.nbr, C.ucoef, blk);
   };
+  auto stalled = [&](int m) { return STALL && m == (n_act - 1) / (int)gridDim.x; };
   auto fetch_w = [&](int blk, int m) {  // w0 of the CTA's m-th block
-    if (tid == 32) {
+    if (tid == 32 && !stalled(m)) {
       async::mbar_expect_tx(&S.wbar[m & 1], BLOCK_CELLS * 8);
       async::bulk_g2s(S.w[m & 1], w0 + (size_t)blk * BLOCK_CELLS, BLOCK_CELLS * 8, &S.wbar[m & 1]);
     }
@@ -272,7 +274,7 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const double* __restrict__
     // Copies that may still be on their way into this CTA's shared memory:
     // block n's and n + 1's records and block n's w0 (a step issues the ones
     // after them only once its waits have succeeded).
-    bool drained = async::mbar_drain(&S.wbar[n & 1], (n >> 1) & 1);
+    bool drained = stalled(n) || async::mbar_drain(&S.wbar[n & 1], (n >> 1) & 1);
     drained = async::mbar_drain(&S.rbar[n % 3], (n / 3) & 1) && drained;
     if (ahead) drained = async::mbar_drain(&S.rbar[(n + 1) % 3], ((n + 1) / 3) & 1) && drained;
     // stop every instance of this CTA's chunk and of its later candidates
@@ -293,7 +295,12 @@ matvec_block_kernel(const __grid_constant__ MixCtx C, const double* __restrict__
 template <int NV, bool JAC>
 void launch(cudaStream_t s, const MixCtx& C, int count, const double* x, const double* A,
             double* y, const double* w0, double omega) {
-  auto kernel = C.gin ? matvec_block_kernel<NV, JAC, PUSHED> : matvec_block_kernel<NV, JAC, PULL>;
+  constexpr bool FIRST = NV < 2;  // a solve's first stencil launch never has two sums
+  auto kernel = C.stall == 2 && FIRST
+                    ? (C.gin ? matvec_block_kernel<NV, JAC, PUSHED, FIRST>
+                             : matvec_block_kernel<NV, JAC, PULL, FIRST>)
+                    : (C.gin ? matvec_block_kernel<NV, JAC, PUSHED, false>
+                             : matvec_block_kernel<NV, JAC, PULL, false>);
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
   kernel<<<count, NT, sizeof(Smem), s>>>(C, x, A, y, w0, omega);
 }

@@ -273,7 +273,7 @@ ffvgpu_status ensure_kpipe(ffvgpu_pool* P) {
   return FFVGPU_OK;
 }
 
-MixCtx krylov_mix_ctx(const ffvgpu_pool* P, int fin) {
+MixCtx krylov_mix_ctx(const ffvgpu_pool* P, int fin, int stall) {
   const int nb = P->nb;
   MixCtx C;
   C.active = P->kpipe + 1;
@@ -290,7 +290,7 @@ MixCtx krylov_mix_ctx(const ffvgpu_pool* P, int fin) {
   C.capacity = nb;
   C.first = 0;
   C.wait_ns = P->wait_ns;
-  C.stall = 0;
+  C.stall = stall;
   C.cf = 0;
   C.depth = 1;
   C.sweep_threads = P->m_sweep_threads;
@@ -304,12 +304,17 @@ MixCtx krylov_mix_ctx(const ffvgpu_pool* P, int fin) {
 struct KrylovForm {
   bool ring = false;
   int grid = 0;
+  int stall = 0;  // test hook (MixCtx::stall)
   double* g[2] = {nullptr, nullptr};
 };
 
 ffvgpu_status krylov_form(ffvgpu_pool* P, KrylovForm* F) {
   ffvgpu_status s;
   if ((s = ring_pool(P, &F->ring)) || (s = ensure_kpipe(P))) return s;
+  if (P->stall_sweep == 2) {  // the test hook covers one solve
+    F->stall = 2;
+    P->stall_sweep = 0;
+  }
   if (F->ring) {
     if (!P->grid_ring) {
       int a, b, c, d;
@@ -331,7 +336,7 @@ ffvgpu_status krylov_form(ffvgpu_pool* P, KrylovForm* F) {
 // (FIN_BI_TS, then FIN_BI_TT) when 'two'.  gin: x's pushed guides (or null).
 void krylov_matvec(ffvgpu_pool* P, const KrylovForm& F, const double* x, double* q,
                    const double* w, int fin, bool two, const double* gin) {
-  MixCtx C = krylov_mix_ctx(P, fin);
+  MixCtx C = krylov_mix_ctx(P, fin, F.stall);
   C.gin = gin;
   if (F.ring)
     launch_mx_matvec(P->stream, C, F.grid, two ? 2 : 1, 0, 0, x, P->A, q, w, true);
@@ -347,7 +352,7 @@ double* krylov_jacobi(ffvgpu_pool* P, const KrylovForm& F, double* const z[2], c
                       int& launches) {
   for (int k = 2; k <= K; ++k) {
     const bool last = k == K;
-    MixCtx C = krylov_mix_ctx(P, dot && last ? FIN_CG_RR1 : 0);
+    MixCtx C = krylov_mix_ctx(P, dot && last ? FIN_CG_RR1 : 0, F.stall);
     C.gin = F.g[k & 1];
     // the vector after CG's last pass is not a stencil's operand (p is)
     C.gout = dot && last ? nullptr : F.g[(k - 1) & 1];

@@ -31,9 +31,10 @@ inline ffvgpu_status bad(const char* why) {
 // (SolveState::timeout_where bits).
 inline std::string timeout_message(int where) {
   std::string m = "a bounded device wait gave up (";
-  const char* names[] = {"producer", "gatherer", "consumer", "sweep", "drain", "A*x"};
+  const char* names[] = {"producer", "gatherer", "consumer", "sweep", "drain", "A*x",
+                         "FP64 A*x or Jacobi pass"};
   bool any = false;
-  for (int b = 0; b < 6; ++b)
+  for (int b = 0; b < 7; ++b)
     if (where & (1 << b)) {
       m += any ? ", " : "";
       m += names[b];

@@ -594,7 +594,7 @@ class Pool:
         _check(lib().ffvgpu_pool_cap_grids(self._h, int(ctas)), "pool_cap_grids")
 
     def stall_next_matvec(self):
-        """Test hook: the next mixed solve's pipelined A*x issues no copy."""
+        """Test hook: the next mixed, CG or BiCGSTAB solve's A*x waits for a copy never issued."""
         _check(lib().ffvgpu_pool_stall_next_matvec(self._h), "pool_stall_next_matvec")
 
     def fill(self, field, value):

@@ -147,8 +147,10 @@ ffvgpu_status ffvgpu_pool_set_wait_limit(ffvgpu_pool* pool, double seconds);
  * that is never issued, so that wait runs out after the wait limit and the
  * solve ends with FFVGPU_TIMEOUT.  The hook covers that one solve. */
 ffvgpu_status ffvgpu_pool_stall_next_solve(ffvgpu_pool* pool);
-/* The same for the pipelined A*x kernel (matvec_form 0): its producer issues
- * no copy, so the consumers' first wait for a slot runs out. */
+/* The same for the A*x of the next mixed solve with the pipelined kernel
+ * (matvec_form 0; its producer issues no copy, so the consumers' first wait for
+ * a slot runs out), or for the A*x and Jacobi kernels of the next FP64 CG or
+ * BiCGSTAB solve (one block's copy is not issued). */
 ffvgpu_status ffvgpu_pool_stall_next_matvec(ffvgpu_pool* pool);
 /* Test hook: the persistent kernels (the mixed form's, and the FP64 CG and
  * BiCGSTAB's A*x and Jacobi sweeps) run at most 'ctas' CTAs (0: SMs x

@@ -39,3 +39,23 @@ def test_rbgs_wait_runs_out(level, kw, varied, count):
     run(g, P, O, "rbgs", (1.1, count, 0.0))
     P.close()
     O.close()
+
+
+# one block a CTA; two; blocks of a list's third chunk (one CTA); the coefficient ring
+@pytest.mark.parametrize("level,ctas,varied", [(2, 0, None), (3, 0, None), (3, 1, None),
+                                               (3, 0, 1.0)])
+@pytest.mark.parametrize("solver,args", [("cg", (1.0, 1, 4, 0.0)), ("cg", (1.0, 3, 4, 0.0)),
+                                         ("bicgstab", (1.0, 1, 4, 0.0)),
+                                         ("bicgstab", (1.0, 2, 4, 0.0))])
+def test_krylov_stencil_wait_runs_out(level, ctas, varied, solver, args):
+    g, inp, O = problem(level)
+    P = device_problem(g, inp)
+    if varied is not None:
+        set_varied(g, P, O, varied)
+    P.cap_grids(ctas)
+    P.stall_next_matvec()
+    times_out(P, lambda: getattr(P, "solve_" + solver)(*args),
+              "A*x" if varied else "FP64 A*x or Jacobi pass")
+    run(g, P, O, solver, args)
+    P.close()
+    O.close()
