@@ -39,6 +39,7 @@ void launch_rbgs(cudaStream_t s, const KCtx& C, bool res, bool sweep, const doub
                  double* xout, const double* A, const double* b, RbgsGuides from,
                  const double* gin, double* gout, double omega, double* partials, SolveState* st,
                  int fin, int iter, bool pdl = false, const int32_t* order = nullptr);
+int rbgs_ordered_blocks();  // pools up to here take an order
 // Test hook: the first sweep (stored guides, no residual), in the form that
 // launch_rbgs or, ring, launch_rbgs_ring would take, with copies left out that
 // it then waits for.

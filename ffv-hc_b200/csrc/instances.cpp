@@ -139,8 +139,7 @@ ffvgpu_status ensure_mixed_buffers(ffvgpu_pool* P, bool d64) {
       (s = dalloc_t(P, &P->me[0], n)) ||
       (s = dalloc_t(P, &P->me[1], n)) || (s = dalloc_t(P, &P->mph, n)) ||
       (s = dalloc_t(P, &P->msh, n)) ||
-      (s = dalloc_t(P, &P->r, n)) || (s = dalloc_t(P, &P->r0, n)) || (s = dalloc_t(P, &P->p, n)) ||
-      (s = dalloc_t(P, &P->q, n)) || (s = dalloc_t(P, &P->sv, n)) || (s = dalloc_t(P, &P->tv, n)))
+      (s = dalloc_vectors(P, {&P->r, &P->r0, &P->p, &P->q, &P->sv, &P->tv})))
     return s;
   if (d64 && ((s = dalloc_t(P, &P->mcoef64, 7 * n)) || (s = dalloc_t(P, &P->me64[0], n)) ||
               (s = dalloc_t(P, &P->me64[1], n)) || (s = dalloc_t(P, &P->mph64, n)) ||

@@ -42,6 +42,22 @@ ffvgpu_status dalloc(ffvgpu_pool* P, void** ptr, size_t bytes) {
   return FFVGPU_OK;
 }
 
+ffvgpu_status dalloc_vectors(ffvgpu_pool* P, std::initializer_list<double**> v) {
+  size_t missing = 0;
+  for (double** p : v) missing += *p == nullptr;
+  if (!missing) return FFVGPU_OK;
+  const size_t n = field_count(P);
+  double* slab = nullptr;
+  ffvgpu_status s = dalloc_t(P, &slab, missing * n);
+  if (s != FFVGPU_OK) return s;
+  P->vector_slabs.push_back(slab);
+  for (double** p : v)
+    if (!*p) {
+      *p = slab;
+      slab += n;
+    }
+  return FFVGPU_OK;
+}
 
 ffvgpu_status ensure_stage(ffvgpu_pool* P, size_t bytes) {
   if (P->stage_bytes >= bytes) return FFVGPU_OK;
@@ -184,11 +200,28 @@ ffvgpu_status require_system(ffvgpu_pool* P) {
   return field_ptr(P, FFVGPU_FIELD_X, true, &xp, &st, nullptr);
 }
 
+// The tables of the FP64 solvers as one allocation.  On small grids much of a
+// pool's first solve is allocations: BiCGSTAB, 128 blocks, 24 iterations, took
+// 6.3 ms on a new pool with one per vector, table and guide buffer, 3.1 with
+// one each for the vectors, the tables and the guides; 2.4 from then on.  (CG,
+// 548 blocks: 8.7, 7.1; 6.3.)
+ffvgpu_status ensure_tables(ffvgpu_pool* P) {
+  if (P->tables) return FFVGPU_OK;
+  const size_t nb = P->nb, doubles = 10 * nb, ints = 3 * nb + 5;
+  ffvgpu_status s = dalloc(P, &P->tables, doubles * sizeof(double) + ints * sizeof(int32_t));
+  if (s != FFVGPU_OK) return s;
+  P->urec = static_cast<double*>(P->tables);
+  P->kpart = P->urec + 8 * nb;
+  P->kraw = reinterpret_cast<int32_t*>(P->kpart + 2 * nb);
+  P->kpipe = P->kraw + nb + 1;
+  P->ucount_d = P->kpipe + 2 * nb + 3;
+  return FFVGPU_OK;
+}
+
 // The uniform records of A (KCtx::urec) when A changed.
 ffvgpu_status ensure_urec(ffvgpu_pool* P) {
   ffvgpu_status s;
-  if ((s = dalloc_t(P, &P->urec, (size_t)P->nb * 8)) || (s = dalloc_t(P, &P->ucount_d, 1)))
-    return s;
+  if ((s = ensure_tables(P))) return s;
   if (P->urec_version != P->sys_version) {
     CK(cudaMemsetAsync(P->ucount_d, 0, sizeof(int32_t), P->stream));
     launch_urec(P->stream, P->nb, P->A, P->urec, P->ucount_d);
@@ -237,31 +270,26 @@ ffvgpu_status ring_pool(ffvgpu_pool* P, bool* ring) {
 // The guide buffers that RBGS passes push into, for a neighbour table in which
 // every face is the other side's neighbour too (a shard's halo faces are not).
 ffvgpu_status ensure_push(ffvgpu_pool* P) {
-  if (!P->nbr_mutual) return FFVGPU_OK;
-  ffvgpu_status s;
+  if (!P->nbr_mutual || P->gpush[0]) return FFVGPU_OK;
   const size_t n = (size_t)P->nb * 6 * FACE_CELLS;
-  if ((s = dalloc_t(P, &P->gpush[0], n))) return s;
-  return dalloc_t(P, &P->gpush[1], n);
+  ffvgpu_status s = dalloc_t(P, &P->gpush[0], 2 * n);
+  if (s == FFVGPU_OK) P->gpush[1] = P->gpush[0] + n;
+  return s;
 }
 
-// The FP64 solvers' pipelined A*x over the pool as one instance: its block
-// list (the blocks that stream their coefficients first, so the persistent
-// grid deals them out evenly), instance tables and per-block sums.
+// The pool as one instance for the FP64 solvers' persistent kernels: its block
+// list (the blocks that stream their coefficients first, so that the grid deals
+// them out evenly) and instance tables.
 ffvgpu_status ensure_kpipe(ffvgpu_pool* P) {
   ffvgpu_status s;
   if ((s = ensure_urec(P))) return s;
   const int nb = P->nb;
-  if (!P->kpipe_ready) {  // allocations already made are kept by dalloc on a retry
-    if ((s = dalloc_t(P, &P->kpipe, (size_t)2 * nb + 3)) ||
-        (s = dalloc_t(P, &P->kraw, (size_t)nb + 1)) ||
-        (s = dalloc_t(P, &P->kpart, (size_t)2 * nb)))
-      return s;
-    std::vector<int32_t> h((size_t)2 * nb + 3, 0);
+  if (!P->kpipe_ready) {
+    std::vector<int32_t> h((size_t)3 * nb + 4, 0);  // kraw, then kpipe
     h[0] = nb;
     for (int b = 0; b < nb; ++b) h[1 + b] = b;
-    h[(size_t)2 * nb + 2] = nb;  // count; blk_inst and first stay 0
-    CK(upload(P, P->kraw, h.data(), sizeof(int32_t) * ((size_t)nb + 1)));
-    CK(upload(P, P->kpipe + 1 + nb, h.data() + 1 + nb, sizeof(int32_t) * ((size_t)nb + 2)));
+    h.back() = nb;  // count; blk_inst and first stay 0, the list is ordered below
+    CK(upload(P, P->kraw, h.data(), sizeof(int32_t) * h.size()));
     P->kpipe_version = 0;
     P->kpipe_ready = true;
   }
@@ -623,13 +651,12 @@ void ffvgpu_pool_destroy(ffvgpu_pool* P) {
   if (P->stream) cudaStreamSynchronize(P->stream);
   if (P->own_stream) cudaStreamSynchronize(P->own_stream);
   release_instances(P);
-  void* ptrs[] = {P->x[0], P->x[1], P->gx, P->A, P->urec, P->ucount_d, P->b, P->u[0], P->u[1], P->u[2],
-                  P->gu[0], P->gu[1], P->gu[2], P->cut, P->vface, P->lapp, P->flags, P->r,
-                  P->p, P->q, P->z[0], P->z[1], P->r0, P->sv, P->tv, P->zb[0], P->zb[1],
-                  P->partials, P->st, P->hist_d, P->kpipe, P->kraw, P->kpart, P->gpush[0], P->gpush[1],
-                  P->stage, P->nbr_d, P->dx_d};
+  void* ptrs[] = {P->x[0], P->x[1], P->gx, P->A, P->tables, P->b, P->u[0], P->u[1], P->u[2],
+                  P->gu[0], P->gu[1], P->gu[2], P->cut, P->vface, P->lapp, P->flags,
+                  P->partials, P->st, P->hist_d, P->gpush[0], P->stage, P->nbr_d, P->dx_d};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  for (void* p : P->vector_slabs) cudaFree(p);
   if (P->host_done) cudaFreeHost(P->host_done);
   for (cudaEvent_t ev : {P->ev0, P->ev1, P->ev2, P->ev3})
     if (ev) cudaEventDestroy(ev);
@@ -981,10 +1008,13 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   double* g[2] = {nullptr, nullptr};
   const int32_t* order = nullptr;
   if (!ring) {
-    if ((s = ensure_push(P)) || (s = ensure_kpipe(P))) return s;
+    if ((s = ensure_push(P))) return s;
     for (int k = 0; k < 2; ++k) g[k] = P->gpush[k];
     if (g[0]) from = RbgsGuides::PUSHED;
-    order = P->kpipe + 1;
+    if (P->nb <= rbgs_ordered_blocks()) {
+      if ((s = ensure_kpipe(P))) return s;
+      order = P->kpipe + 1;
+    }
   }
   const KCtx C = P->ctx(P->bc_p);
   const int every = prm->check_every > 0 ? prm->check_every : 32;
@@ -1157,10 +1187,7 @@ ffvgpu_status ffvgpu_solve_cg(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   cudaSetDevice(P->device);
   ffvgpu_status s;
   if ((s = require_system(P))) return s;
-  const size_t n = field_count(P);
-  if ((s = dalloc_t(P, &P->r, n)) || (s = dalloc_t(P, &P->p, n)) || (s = dalloc_t(P, &P->q, n)) ||
-      (s = dalloc_t(P, &P->z[0], n)) || (s = dalloc_t(P, &P->z[1], n)))
-    return s;
+  if ((s = dalloc_vectors(P, {&P->r, &P->p, &P->q, &P->z[0], &P->z[1]}))) return s;
   const int N = prm->count_max;
   ffvgpu_result R;
   std::memset(&R, 0, sizeof(R));
@@ -1272,11 +1299,8 @@ ffvgpu_status ffvgpu_solve_bicgstab(ffvgpu_pool* P, const ffvgpu_iter_params* pr
   cudaSetDevice(P->device);
   ffvgpu_status s;
   if ((s = require_system(P))) return s;
-  const size_t n = field_count(P);
-  if ((s = dalloc_t(P, &P->r, n)) || (s = dalloc_t(P, &P->r0, n)) || (s = dalloc_t(P, &P->p, n)) ||
-      (s = dalloc_t(P, &P->q, n)) || (s = dalloc_t(P, &P->sv, n)) || (s = dalloc_t(P, &P->tv, n)) ||
-      (s = dalloc_t(P, &P->z[0], n)) || (s = dalloc_t(P, &P->z[1], n)) ||
-      (s = dalloc_t(P, &P->zb[0], n)) || (s = dalloc_t(P, &P->zb[1], n)))
+  if ((s = dalloc_vectors(P, {&P->r, &P->r0, &P->p, &P->q, &P->sv, &P->tv, &P->z[0], &P->z[1],
+                              &P->zb[0], &P->zb[1]})))
     return s;
   const int N = prm->count_max;
   ffvgpu_result R;

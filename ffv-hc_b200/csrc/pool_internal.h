@@ -3,6 +3,7 @@
 // batches of independent problems and the mixed-precision form).
 #pragma once
 #include <cstdint>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -93,6 +94,9 @@ struct ffvgpu_pool {
   int xcur = 0;
   double* gx = nullptr;  // stored first guide layer of x
   double* A = nullptr;   // [nb][7][4096]
+  // the FP64 solvers' tables, one allocation (ensure_tables): urec, kpart, kpipe,
+  // kraw and ucount_d point into it
+  void* tables = nullptr;
   double* urec = nullptr;         // [nb][8] uniform records of A (launch_urec)
   int32_t* ucount_d = nullptr;    // uniform blocks
   int32_t ucount_h = 0;           // the same, read back for a solve's byte count
@@ -106,6 +110,8 @@ struct ffvgpu_pool {
   double* vface = nullptr;  // [6][nb*4096]
   double* lapp = nullptr;   // Laplacian of p (bcut_corr_u)
   uint8_t* flags = nullptr; // bits 0..5 cut ids, bit 7 fluid
+  // vectors of the Krylov solvers and the mixed form (dalloc_vectors)
+  std::vector<void*> vector_slabs;
   double* r = nullptr;
   double* p = nullptr;
   double* q = nullptr;
@@ -121,7 +127,7 @@ struct ffvgpu_pool {
   void* stage = nullptr;
   size_t stage_bytes = 0;
   int32_t* host_done = nullptr;  // pinned
-  // the FP64 solvers' pipelined A*x: the pool as one instance.  kpipe:
+  // the FP64 solvers' A*x and Jacobi passes: the pool as one instance.  kpipe:
   // [1 + nb] the block list (count, then the blocks that stream their
   // coefficients first), [nb] instance of each block (0), then first (0) and
   // count (nb); kraw: the list in block order; kpart: [2][nb] per-block sums
@@ -130,8 +136,10 @@ struct ffvgpu_pool {
   double* kpart = nullptr;
   int64_t kpipe_version = 0;  // sys_version the list was ordered for
   bool nbr_mutual = false;  // every face is the other side's neighbour too
-  double* gpush[2] = {nullptr, nullptr};  // [nb][6][256] guides pushed by RBGS passes
-  bool kpipe_ready = false;   // all three allocated and the tables uploaded
+  // [nb][6][256] each, one allocation: guides pushed by RBGS passes and by the
+  // Krylov solvers' steps and Jacobi passes
+  double* gpush[2] = {nullptr, nullptr};
+  bool kpipe_ready = false;   // kpipe and kraw uploaded
 
   // instances: a pool made from one grid is instance 0 over every block; a
   // batch pool admits and releases instances over its block capacity
@@ -232,6 +240,9 @@ template <class T>
 ffvgpu_status dalloc_t(ffvgpu_pool* P, T** ptr, size_t count) {
   return dalloc(P, reinterpret_cast<void**>(ptr), count * sizeof(T));
 }
+// Vectors of one value per cell that the pool does not have yet, as one
+// allocation in P->vector_slabs.
+ffvgpu_status dalloc_vectors(ffvgpu_pool* P, std::initializer_list<double**> v);
 ffvgpu_status ensure_stage(ffvgpu_pool* P, size_t bytes);
 // The values of a host buffer (bytes long) as the pack kernel reads them: the
 // buffer itself when it is pinned host memory the device can address (the

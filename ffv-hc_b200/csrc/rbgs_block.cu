@@ -339,14 +339,8 @@ void launch_one(cudaStream_t s, const KCtx& C, const double* xin, double* xout, 
   const int grid = std::min(C.nb, 2 * sms);
   auto kernel = one ? rbgs_block_kernel<R, W, G, 1, STALL> : rbgs_block_kernel<R, W, G, 2, STALL>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
-  // With up to twelve blocks per SM the varied blocks, which take three times as
-  // long, go first so that none is left for the end; with more the order mixes
-  // them, so that one CTA's coefficient loads overlap the other's arithmetic.
-  // us per pass, varied first / block order, by blocks per SM: 2.2: 24.0 / 29.0,
-  // 3.7: 34.4 / 35.8, 4.8: 45.8 / 53.7, 7.9: 59.5 / 68.6, 11.3: 74.5 / 77.9,
-  // 15.3: 107.6 / 106.2, 21: 108.2 / 105.5, 32: 158.4 / 147.9.
   launch_dep(kernel, grid, NT, sizeof(Smem), s, pdl, C, xin, xout, A, b, gst, gout, omega,
-             partials, st, fin, iter, C.nb <= 12 * sms ? order : nullptr);
+             partials, st, fin, iter, order);
 }
 
 }  // namespace
@@ -362,6 +356,14 @@ int sm_count() {
   if (n == 0) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
   return n > 0 ? n : 1;
 }
+
+// With up to twelve blocks per SM the varied blocks, which take three times as
+// long, go first so that none is left for the end; with more the order mixes
+// them, so that one CTA's coefficient loads overlap the other's arithmetic.
+// us per pass, varied first / block order, by blocks per SM: 2.2: 24.0 / 29.0,
+// 3.7: 34.4 / 35.8, 4.8: 45.8 / 53.7, 7.9: 59.5 / 68.6, 11.3: 74.5 / 77.9,
+// 15.3: 107.6 / 106.2, 21: 108.2 / 105.5, 32: 158.4 / 147.9.
+int rbgs_ordered_blocks() { return 12 * sm_count(); }
 
 void launch_rbgs_stalled(cudaStream_t s, const KCtx& C, bool ring, const double* xin,
                          double* xout, const double* A, const double* b, const double* gin,
