@@ -267,14 +267,17 @@ ffvgpu_status ring_pool(ffvgpu_pool* P, bool* ring) {
   return FFVGPU_OK;
 }
 
-// The guide buffers that RBGS passes push into, for a neighbour table in which
-// every face is the other side's neighbour too (a shard's halo faces are not).
-ffvgpu_status ensure_push(ffvgpu_pool* P) {
-  if (!P->nbr_mutual || P->gpush[0]) return FFVGPU_OK;
+// The guide buffers that the FP64 solvers' kernels push into, for a neighbour
+// table in which every face is the other side's neighbour too (a shard's halo
+// faces are not).  Without room for them (24 KB a block) the kernels take their
+// guides from the neighbours' interiors, with the same results.
+void ensure_push(ffvgpu_pool* P) {
+  if (!P->nbr_mutual || P->gpush[0]) return;
   const size_t n = (size_t)P->nb * 6 * FACE_CELLS;
-  ffvgpu_status s = dalloc_t(P, &P->gpush[0], 2 * n);
-  if (s == FFVGPU_OK) P->gpush[1] = P->gpush[0] + n;
-  return s;
+  if (dalloc_t(P, &P->gpush[0], 2 * n) == FFVGPU_OK)
+    P->gpush[1] = P->gpush[0] + n;
+  else
+    cudaGetLastError();  // not a failure of the solve
 }
 
 // The pool as one instance for the FP64 solvers' persistent kernels: its block
@@ -352,7 +355,7 @@ ffvgpu_status krylov_form(ffvgpu_pool* P, KrylovForm* F) {
   } else {
     if (!P->grid_krylov) P->grid_krylov = matvec_block_grid();
     F->grid = P->grid_krylov;
-    if ((s = ensure_push(P))) return s;
+    ensure_push(P);
     F->g[0] = P->gpush[0];
     F->g[1] = P->gpush[1];
   }
@@ -1008,7 +1011,7 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   double* g[2] = {nullptr, nullptr};
   const int32_t* order = nullptr;
   if (!ring) {
-    if ((s = ensure_push(P))) return s;
+    ensure_push(P);
     for (int k = 0; k < 2; ++k) g[k] = P->gpush[k];
     if (g[0]) from = RbgsGuides::PUSHED;
     if (P->nb <= rbgs_ordered_blocks()) {
