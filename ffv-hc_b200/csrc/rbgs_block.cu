@@ -58,6 +58,7 @@ struct Uniform {
 };
 struct Varied {
   const double* Ab;  // at the thread's first cell
+  __device__ __forceinline__ explicit Varied(const double* A, bool = true) : Ab(A) {}
   __device__ __forceinline__ K7 at(int c, int n) const {
     return stream_coefs(Ab, c * HALF_CELLS + plane(n) * 128);
   }
@@ -72,9 +73,12 @@ struct Varied {
 struct Held {
   const double* Ab;
   K7 k1[NC];
-  __device__ __forceinline__ explicit Held(const double* A) : Ab(A) {
+  // (a uniform block, which does not use them, loads none: its pass would read
+  // 115 KB more)
+  __device__ __forceinline__ Held(const double* A, bool varied) : Ab(A), k1() {
+    if (varied)
 #pragma unroll
-    for (int n = 0; n < NC; ++n) k1[n] = stream_coefs(Ab, HALF_CELLS + plane(n) * 128);
+      for (int n = 0; n < NC; ++n) k1[n] = stream_coefs(Ab, HALF_CELLS + plane(n) * 128);
   }
   __device__ __forceinline__ K7 at(int c, int n) const {
     return c ? k1[n] : stream_coefs(Ab, plane(n) * 128);
@@ -233,7 +237,9 @@ rbgs_block_kernel(const __grid_constant__ KCtx C, const double* xin,
   // a limit of 0 lets nothing be waited for: the pass gives up here, whether or
   // not the record happens to have landed by the time a wait would look
   bool ok = blk < 0 || C.wait_ns != 0;
-  std::conditional_t<PER_SM == 1, Held, Varied> AV{A + (size_t)blk * 7 * BLOCK_CELLS + slot(tid)};
+  std::conditional_t<PER_SM == 1, Held, Varied> AV(
+      A + (size_t)blk * 7 * BLOCK_CELLS + slot(tid),
+      PER_SM == 1 && __ldg(C.urec + (size_t)blk * 8 + 7) == 0.0);
   pdl_release();
   pdl_wait();
   const bool skip = *((volatile const int32_t*)&st->done) != 0;  // used after the first wait
