@@ -26,9 +26,10 @@ struct KCtx {
   const double* urec;
 };
 
-// Where a pass takes its blocks' guide layers from: stored (gin [blk][face][p]),
-// the neighbours' interiors, or the neighbours' interiors with what the sweep
-// before pushed into gin.
+// Where a pass takes its blocks' guide layers from: stored (gin [blk][face][p];
+// not with sweep and residual together), the neighbours' interiors, or the
+// neighbours' interiors with what the sweep before pushed into gin (only with
+// the residual).
 enum class RbgsGuides { STORED, PULL, PUSHED };
 // Fused residual + red-black sweep (rbgs_block.cu); C.urec must be set.  A
 // sweep with gout pushes guides for the next pass into it (PUSHED).
@@ -59,11 +60,11 @@ int sm_count();  // of the current device
 // every cell has those seven coefficients, else 0.0), adding the uniform
 // blocks to *ucount.
 void launch_urec(cudaStream_t s, int nb, const double* A, double* urec, int32_t* ucount);
-// Jacobi sweep from the zero field (the preconditioner's first pass); a
-// block with a set uniform record (C.urec) reads its seven coefficients from
-// it.  dot: also b.x1 (FIN_CG_RR1).
-void launch_jacobi(cudaStream_t s, const KCtx& C, bool dot, double* xout, const double* A,
-                   const double* b, double omega, double* partials, SolveState* st);
+// Jacobi sweep from the zero field, with b.x1 (FIN_CG_RR1): CG's preconditioner
+// of one pass.  A block with a set uniform record (C.urec) reads its seven
+// coefficients from it.
+void launch_jacobi_dot(cudaStream_t s, const KCtx& C, double* xout, const double* A,
+                       const double* b, double omega, double* partials, SolveState* st);
 void launch_calc_r(cudaStream_t s, const KCtx& C, const double* x, const double* gst,
                    const double* A, const double* b, double* r, SolveState* st);
 // Cell-wise steps of the Krylov solvers (krylov_block.cu), with the Jacobi pass

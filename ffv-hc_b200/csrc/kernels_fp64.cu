@@ -132,16 +132,15 @@ __device__ void reduce_finalize(const double (&acc)[2][2], double* __restrict__ 
 
 // ---------------------------------------------------------------------------
 // Jacobi smoother (bils.f90:5-55) from the zero field of FFVILS::Fill(z, 0)
-// (blas.f90:5-33, guides included) with b = bvec: the first pass of
-// Jacobi_PreConditioner.  Later passes read a stored iterate and run on the
-// pipelined kernel (launch_jacobi_pipe).  DOT: also forms b.x1
-// (FFVILS.h:712-718 DOT(r, z), r = bvec).  Every neighbour is 0.0, and the
-// products with it are kept, so the result has the reference's bits (the
-// sign of a zero residual included).  A block whose uniform record
+// (blas.f90:5-33, guides included) with b = bvec, and b.x1 (FFVILS.h:712-718
+// DOT(r, z), r = bvec): CG's preconditioner where it is one pass (with more,
+// the first comes with the step that makes r, krylov_block.cu).  Every
+// neighbour is 0.0, and the products with it are kept, so the result has the
+// reference's bits (the sign of a zero residual included).  A block whose uniform record
 // (KCtx::urec) is set has the same seven coefficients in every cell: they
 // are read once from the record, and the block moves b and x only.
 // ---------------------------------------------------------------------------
-template <bool DOT, bool UNI>
+template <bool UNI>
 __device__ __forceinline__ void jacobi_cells(const double* __restrict__ Ab,
                                              const double* __restrict__ ur,
                                              const double* __restrict__ bb, double* __restrict__ xo,
@@ -166,12 +165,11 @@ __device__ __forceinline__ void jacobi_cells(const double* __restrict__ Ab,
       const double x_tmp = r / coef(0, s);
       const double x1 = x0 - omega * (x0 - x_tmp);
       xo[s] = x1;
-      if (DOT) acc[c][m & 1] += bv * x1;
+      acc[c][m & 1] += bv * x1;
     }
   }
 }
 
-template <bool DOT>
 __global__ void __launch_bounds__(THREADS, 3)
 jacobi_kernel(KCtx C, double* __restrict__ xout, const double* __restrict__ A,
               const double* __restrict__ bvec, double omega, double* __restrict__ partials,
@@ -185,10 +183,10 @@ jacobi_kernel(KCtx C, double* __restrict__ xout, const double* __restrict__ A,
   double* xo = xout + (size_t)blk * BLOCK_CELLS;
   double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
   if (uni)
-    jacobi_cells<DOT, true>(Ab, ur, bb, xo, omega, acc);
+    jacobi_cells<true>(Ab, ur, bb, xo, omega, acc);
   else
-    jacobi_cells<DOT, false>(Ab, ur, bb, xo, omega, acc);
-  if (DOT) reduce_finalize(acc, partials, st, FIN_CG_RR1, 0);
+    jacobi_cells<false>(Ab, ur, bb, xo, omega, acc);
+  reduce_finalize(acc, partials, st, FIN_CG_RR1, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -682,12 +680,9 @@ fill_kernel(double* __restrict__ x, size_t stride, double* __restrict__ g, doubl
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
-void launch_jacobi(cudaStream_t s, const KCtx& C, bool dot, double* xout, const double* A,
-                   const double* b, double omega, double* partials, SolveState* st) {
-  if (dot)
-    jacobi_kernel<true><<<C.nb, THREADS, 0, s>>>(C, xout, A, b, omega, partials, st);
-  else
-    jacobi_kernel<false><<<C.nb, THREADS, 0, s>>>(C, xout, A, b, omega, partials, st);
+void launch_jacobi_dot(cudaStream_t s, const KCtx& C, double* xout, const double* A,
+                       const double* b, double omega, double* partials, SolveState* st) {
+  jacobi_kernel<<<C.nb, THREADS, 0, s>>>(C, xout, A, b, omega, partials, st);
 }
 
 void launch_calc_r(cudaStream_t s, const KCtx& C, const double* x, const double* gst,

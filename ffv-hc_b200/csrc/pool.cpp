@@ -1241,7 +1241,7 @@ ffvgpu_status ffvgpu_solve_cg(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
     // z = Jacobi^K(0) with b = r; the last pass also forms r.z.  The pass from
     // zero comes with the update of r (K > 1), or is the only one
     if (K == 1) {
-      launch_jacobi(P->stream, C, true, P->z[0], P->A, P->r, prm->omega, P->partials, P->st);
+      launch_jacobi_dot(P->stream, C, P->z[0], P->A, P->r, prm->omega, P->partials, P->st);
       words += 9;
       coef += 7;
       launches++;

@@ -389,17 +389,16 @@ void launch_rbgs(cudaStream_t s, const KCtx& C, bool res, bool sweep, const doub
                  int fin, int iter, bool pdl, const int32_t* order) {
 #define RBGS(R, W, G) \
   launch_one<R, W, G>(s, C, xin, xout, A, b, gin, gout, omega, partials, st, fin, iter, pdl, order)
-#define RBGS_FROM(R, W)                                     \
-  from == RbgsGuides::STORED ? RBGS(R, W, tile::STORED)     \
-  : from == RbgsGuides::PULL ? RBGS(R, W, tile::PULL)       \
-                             : RBGS(R, W, tile::PUSHED)
+  // stored guides are those before a solve's first sweep, pushed ones those of
+  // the sweep before
   if (res && sweep)
-    RBGS_FROM(true, true);
+    from == RbgsGuides::PUSHED ? RBGS(true, true, tile::PUSHED) : RBGS(true, true, tile::PULL);
   else if (sweep)
-    RBGS_FROM(false, true);
+    from == RbgsGuides::STORED ? RBGS(false, true, tile::STORED) : RBGS(false, true, tile::PULL);
   else
-    RBGS_FROM(true, false);
-#undef RBGS_FROM
+    from == RbgsGuides::STORED ? RBGS(true, false, tile::STORED)
+    : from == RbgsGuides::PULL ? RBGS(true, false, tile::PULL)
+                               : RBGS(true, false, tile::PUSHED);
 #undef RBGS
 }
 
