@@ -231,7 +231,7 @@ __device__ __forceinline__ double outer_guide(double x0, int face, const BCSet& 
 
 // Two guide cells (layer 1) of the same face, positions p0 and p1 in
 // [0, 256) (p = v*16 + u), with every load of both issued before any is
-// used: the batched form of guide_value for the pipelined kernels.  Same
+// used: the batched form of guide_value.  Same
 // expressions, same evaluation order, same results as guide_value.
 template <typename LD = ReadOnly, typename T>
 __device__ __forceinline__ void guide_pair(const T* x, int blk, int face, int p0, int p1,

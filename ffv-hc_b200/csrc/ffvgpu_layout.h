@@ -82,7 +82,7 @@ struct SolveState {
   double best;       // mixed form: smallest residual of the current cycle
   double growth;     // mixed form: restart when the residual exceeds growth * best (0: never)
   double scale;      // RBGS_WithFixedAverage: the cell count the sum is divided by
-  uint32_t work;     // RBGS pass: blocks handed out beyond each CTA's first
+  uint32_t work;     // RBGS pass: blocks handed out beyond each CTA's first two
   int32_t max_cycle; // mixed form: restart after this many iterations of a cycle (0: never)
   int32_t ublocks;   // mixed form: blocks whose seven coefficients are the same in every cell
 };

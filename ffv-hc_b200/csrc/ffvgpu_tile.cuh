@@ -15,10 +15,6 @@
 namespace ffvgpu {
 namespace tile {
 
-// Per colour [k + 1][j + 1][i >> 1] with rows of 8 values, k and j in -1..16:
-// every neighbour of a cell is at a fixed offset, the j- and k-face guides
-// included; the x-face guides sit in two arrays of their own, [face][j + 16 k].
-// With rows of 8 the two rows a half-warp reads fall into disjoint banks.
 // Per colour and plane k in -1..16: rows j = -1..16 of 8 values (i >> 1), then
 // 16 x-face guides, one per row -- of the two guide cells beside a row one has
 // each colour, so a row of one colour has just one of them, west (i = -1) when

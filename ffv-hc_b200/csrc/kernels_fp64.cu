@@ -328,7 +328,8 @@ exchange_kernel(const __grid_constant__ KCtx C, const double* __restrict__ x,
 // block needs are read whole and in the order they lie in: of each plane
 // k = 0..15 the rows j = 0..15 (with guides -1..16), and with guides the same
 // rows of planes -1 and 16 -- runs of at least 16 w doubles, V of them per load,
-// every load in flight before the first store.  The link moves 32-byte
+// the loads of 4096 doubles (vc = 2: of 5120, with guides 6400) in flight
+// before their first store.  The link moves 32-byte
 // sectors, so a row's 16 interior values, 16 bytes into it, cost all of its 160
 // (vc = 2) anyway.  They go through shared memory to their places.
 // 1164 blocks, vc = 2, pinned: with guides 1837 -> 1285 us (59.6 MB, 46 GB/s; read

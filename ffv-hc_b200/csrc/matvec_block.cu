@@ -1,6 +1,7 @@
 // matvec_block.cu -- A x with its dot products, and a Jacobi pass, for sm_100a:
 // the stencil kernels of the FP64 Krylov solvers (FFVILS::CG and BiCGSTAB,
-// src/FFV/FFVILS.h:661-974).
+// src/FFV/FFVILS.h:661-974) on pools of mostly uniform blocks (ring_pool in
+// pool.cpp).
 //
 // y = A x (calc_ax, src/CGMfuncs/bils.f90:162-206) with y.w0 (NV 1: q_.r0 or
 // q.p) or y.w0 and y.y (NV 2: t_.s and t_.t_); or, JAC, a Jacobi sweep of x with

@@ -1037,9 +1037,9 @@ ffvgpu_status ffvgpu_solve_rbgs(ffvgpu_pool* P, const ffvgpu_iter_params* prm,
   launches++;
   CK(cudaEventRecord(P->ev2, P->stream));
   int swept = 0;
-  // Each pass is a programmatic dependent of the pass before it (it
-  // prefetches coefficients during that pass's tail), except where a host
-  // poll or a timing event sits between them.
+  // Each pass is a programmatic dependent of the pass before it (its prologue
+  // and its first records and right-hand sides overlap that pass's tail), except
+  // where a host poll or a timing event sits between them.
   bool polled_last = true;
   for (int n = 2; n <= N; ++n) {
     rbgs_pass(P, ring, C, true, true, P->x[(c0 + n - 1) & 1], P->x[(c0 + n) & 1], from, g[n & 1],

@@ -15,11 +15,12 @@
 // into L2.  What bounds it: the loads and barriers between a block's phases
 // (staging, colour-1 residual, colour 0, colour 1) and shared memory, which
 // the second CTA overlaps only in part; FP64 arithmetic is a quarter of the
-// time.  Level-5 sphere grid (4692 blocks, 4256 uniform), per pass: 238 us for
-// a persistent kernel with one cell per consumer thread and stencil
-// neighbours chosen by selects (500 MB of coefficients and b through a TMA
-// ring), 147 us here; a copy of x through the same structure takes 86 us, the
-// pass without guide layers 125 us.  72 blocks: 18.0 -> 13.7 us; 324: 33 ->
+// time.  Level-5 sphere grid (4692 blocks, 4256 uniform), per pass: 147 us (87
+// at the measured 6463 GB/s for the 561 MB that must move), 230 us with one cell
+// per consumer thread and neighbours chosen by selects (rbgs_ring.cu, which
+// brings 254 MB of coefficients and b through a ring; it serves the pools of
+// mostly varied blocks); a copy of x through the same structure takes 86 us,
+// the pass without guide layers 125 us.  72 blocks: 18.0 -> 13.7 us; 324: 33 ->
 // 25.7 us.  Tried and slower at level 5 (us per pass): 128 threads with whole
 // k columns in registers 199; 512 threads on strided planes, one CTA per SM
 // with everything staged a block ahead 180, two CTAs 163; guides of x and 2:1
