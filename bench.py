@@ -136,7 +136,8 @@ def profile_traffic(level, cells, fmt_bytes):
             return val, f"ncu, {os.path.basename(path)}"
         if fields.get("format_bytes_per_launch"):
             return (val * fmt_bytes / fields["format_bytes_per_launch"],
-                    f"ncu level-{lv} capture scaled by the format bytes")
+                    f"ncu level-{lv} capture (reads measured, x_out counted as written) scaled "
+                    "by the format bytes")
         if fields.get("cells_per_launch"):
             return val * cells / fields["cells_per_launch"], f"ncu level-{lv} capture scaled by cells"
     return None, None
